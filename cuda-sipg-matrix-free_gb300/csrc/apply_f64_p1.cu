@@ -2,6 +2,7 @@
 // launches (element-per-thread and per-node tiles) and batched ones.  One
 // translation unit per precision and degree, so the build compiles them in
 // parallel.
+#include "sipg_apply_fx.cuh"
 #include "sipg_apply_pernode.cuh"
 namespace sipg {
 cudaError_t launch_apply_f64_p1(const TileCfg& cfg, int mode, const ApplyArgs<double>& a, const HostTables& h,

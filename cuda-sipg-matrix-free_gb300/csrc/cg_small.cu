@@ -76,10 +76,10 @@ __device__ double sum_partials(const double* part, int n, double* red_sh, double
 
 template <int P, int SHAPE>
 __global__ void __launch_bounds__(PernodeShape<P, SHAPE>::NT)
-    k_cg_small(const __grid_constant__ SmallCgArgs g, const __grid_constant__ Tab<double, P> tb) {
+    k_cg_small(const __grid_constant__ SmallCgArgs g, const __grid_constant__ ApplyTab<double, P> tb) {
   using S = PernodeShape<P, SHAPE>;
   constexpr int N1 = S::N1, NN = S::NN, EX = S::EX, EY = S::EY, NE = S::NE, NT = S::NT;
-  __shared__ PernodeSmem<double, P, SHAPE> sm;
+  __shared__ PernodeFxSmem<P, SHAPE> sm;
   __shared__ double red_sh[32];
   __shared__ double sc;
   const int t = threadIdx.x;
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(PernodeShape<P, SHAPE>::NT)
   const int dim = g.dim;
   const size_t noe = (size_t)dim * dim;
   const int tiles_x = (dim + EX - 1) / EX, ntiles = tiles_x * ((dim + EY - 1) / EY);
-  pernode_tables<double, P, SHAPE>(sm, tb);
+  pernode_fx_tables<P, SHAPE>(sm, tb.fx, g.nu);
 
   CgState<double> st = *g.st;  // the same copy in every CTA from here on
   ApplyArgs<double> a{};
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(PernodeShape<P, SHAPE>::NT)
     double acc = 0.0;
     for (int tile = blockIdx.x; tile < ntiles; tile += nb) {
       const int x0 = (tile % tiles_x) * EX, y0 = (tile / tiles_x) * EY;
-      acc += pernode_tile<double, P, SHAPE, APPLY_CG, true>(a, sm, x0, y0, st.first != 0, st.beta, pold, pnew);
+      acc += pernode_tile_fx<P, SHAPE, APPLY_CG, true>(a, sm, tb, x0, y0, st.first != 0, st.beta, pold, pnew);
     }
     const double bt = block_sum<double, NT>(acc, red_sh);
     if (t == 0) g.part_a[blockIdx.x] = bt;
@@ -187,7 +187,7 @@ cudaError_t launch_cg_small_shape(const SmallCgArgs& g, const HostTables& h, cud
   // tile and one partial slot each
   const int grid = (int)std::max<long long>(1, std::min<long long>({ntiles, (long long)sms * per_sm,
                                                                     (long long)kSmallCgMaxBlocks}));
-  const Tab<double, P> tb = make_tab<double, P>(h);
+  const ApplyTab<double, P>& tb = apply_tabs<double, P>(h);
   void* args[] = {(void*)&g, (void*)&tb};
   e = cudaLaunchCooperativeKernel((const void*)k, dim3(grid), dim3(S::NT), args, 0, s);
   count_launch();

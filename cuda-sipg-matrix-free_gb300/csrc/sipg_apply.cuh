@@ -1,4 +1,6 @@
-// sipg_apply.cuh -- the fused SIPG-SEM operator apply for sm_103a.
+// sipg_apply.cuh -- the fused SIPG-SEM operator apply for sm_103a: the FP32
+// tile, the launches of both precisions (the FP64 tile: sipg_apply_fx.cuh), and
+// the reductions they share.
 //
 // One kernel computes y = A u for a TX x TY tile of elements per CTA (one
 // thread per element): the tensor-product LGL volume term, the lifting of the
@@ -29,7 +31,7 @@
 //      (store, and in the CG modes a deterministic grid reduction).
 #pragma once
 
-#include "sipg_internal.cuh"
+#include "sipg_fx.cuh"
 
 namespace sipg {
 
@@ -90,9 +92,7 @@ __device__ __forceinline__ bool grid_sum_last(A block_total, const ReduceScratch
 
 // Where the column form reads its weighted stiffness KW (n^3 values): from
 // the kernel parameters (constant bank), or from shared memory where the
-// table read with a per-row index overflows the constant cache.  Measured
-// for FP64 at ~16 M DoF: shared memory pays at p = 8 (5.8 KB; 15.8 -> 17.0
-// GDoF/s), not at p = 6 or 7 (2.7 and 4 KB).
+// table overflows the constant cache.
 template <typename T, int P>
 struct KwInSmem {
   static constexpr bool value = P >= 8;
@@ -119,17 +119,12 @@ struct ApplySmem {
   static constexpr size_t bytes = (size_t)(US + XF + YF + KW) * sizeof(T);
 };
 
-// Phase-2 form per (precision, degree): the column form for FP64 (whose n^2
-// outputs would not fit in registers beyond small p, and whose FP64 pipe is
-// the bottleneck anyway), the all-register form for FP32 up to p = 6.
+// Phase-2 form per degree: the all-register form up to p = 6, the column form
+// beyond (whose n^2 outputs would not fit in registers).
 template <typename T, int P>
 struct ApplyColumnForm {
-  static constexpr bool value = (sizeof(T) == 8) || (P >= 7);
-  // Unroll limits that keep FP64 at high degree out of register spills: the
-  // phase-0 load batch, the halo face loop, and the phase-2 column loop.
-  static constexpr int load_unroll = (sizeof(T) == 8 && P >= 5) ? 2 * (P + 1) : (P + 1) * (P + 1);
-  static constexpr int halo_unroll = (sizeof(T) == 8 && P >= 5) ? 1 : (P + 1);
-  static constexpr int col_unroll = (sizeof(T) == 8 && P >= 5) ? 1 : (P + 1);
+  static constexpr bool value = P >= 7;
+  static constexpr int load_unroll = (P + 1) * (P + 1), halo_unroll = P + 1, col_unroll = P + 1;
 };
 
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
@@ -202,16 +197,14 @@ __device__ __forceinline__ void apply_tile(const ApplyArgs<T>& a, const Tab<T, P
   constexpr int N = P, N1 = P + 1, NN = N1 * N1, TE = TX * TY;
   constexpr bool kCols = ApplyColumnForm<T, P>::value;
   constexpr int BASE = apply_base_mode(MODE);
-  // FP32 (and the FP64 *_PIVOT modes): every sum whose coefficients add up to zero (a derivative row D, a
+  // Every sum whose coefficients add up to zero (a derivative row D, a
   // stiffness row K = D^T W D) is taken over differences from one value of
   // the line, v_i - v_0, which leaves it unchanged in exact arithmetic and
   // drops the part common to the line exactly.  Rounding then scales with
   // the variation of u across an element (h |grad u|), not with u itself: on
   // a smooth vector the FP32 operator's relative error falls from
   // ~kappa eps_32 (~1 at 512 x 512, p = 6) to ~dim eps_32, which is what an
-  // FP32 inner solve needs to see the smooth modes.  (The other FP64 modes
-  // keep the plain sums: their results stay bit-identical to the unpivoted
-  // kernel's.)
+  // FP32 inner solve needs to see the smooth modes.
   constexpr bool kPivot = sizeof(T) == 4 || MODE != BASE;
   using S = ApplySmem<T, P, TX, TY>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -574,10 +567,76 @@ __device__ __forceinline__ void apply_tile(const ApplyArgs<T>& a, const Tab<T, P
   }
 }
 
+// The tables an apply kernel takes: for FP64 the fixed-point ones beside the
+// plain ones of the tiles out of their range.
+template <typename T, int P>
+struct ApplyTab {
+  Tab<T, P> t;
+};
+template <int P>
+struct ApplyTab<double, P> {
+  Tab<double, P> t;
+  FxTab<P> fx;
+};
+
+// The tables of degree P, built once per process (they depend on P alone).
+template <typename T, int P>
+const ApplyTab<T, P>& apply_tabs(const HostTables& h) {
+  static const ApplyTab<T, P> t = [&] {
+    ApplyTab<T, P> v;
+    v.t = make_tab<T, P>(h);
+    if constexpr (sizeof(T) == 8) v.fx = make_fxtab<P>(h);
+    return v;
+  }();
+  return t;
+}
+
+// Shared memory of the fixed-point tile: the elements' parity-form values
+// [NN][TE]; w times their four faces' normal derivatives [4][N1][RS] (LEFT,
+// RIGHT, DOWN, UP), each with the one of the TX or TY elements around the tile
+// that meet it there behind the tile's TE; those elements' traces [N1][HALO].
+template <int P, int TX, int TY>
+struct FxSmem {
+  static constexpr int N1 = P + 1, NN = N1 * N1, TE = TX * TY, HALO = 2 * TX + 2 * TY;
+  static constexpr int RS = TE + (TX > TY ? TX : TY);
+  static constexpr size_t bytes = (size_t)(NN * TE + 4 * N1 * RS + N1 * HALO) * 8;
+};
+
+template <typename T, int P, int TX, int TY>
+constexpr size_t apply_smem() {
+  if constexpr (sizeof(T) == 8) return FxSmem<P, TX, TY>::bytes;
+  else return ApplySmem<T, P, TX, TY>::bytes;
+}
+
+// Resident CTAs the kernel's registers are limited for (0: no limit): in FP64
+// what its shared memory allows, at 64 registers a thread or more.
+template <typename T, int P, int TX, int TY>
+constexpr int apply_min_blocks() {
+  if constexpr (sizeof(T) == 8) {
+    const int smem = (int)((227 * 1024) / (FxSmem<P, TX, TY>::bytes + 2048));
+    const int regs = 65536 / (TX * TY * (P == 1 ? 64 : (P == 2 ? 80 : 128)));
+    const int m = smem < regs ? smem : regs;
+    return m < 1 ? 1 : m;
+  }
+  return 0;
+}
+
+// One CTA's work in FP64: the sums in fixed point (sipg_apply_fx.cuh).
+template <int P, int TX, int TY, int MODE>
+__device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const ApplyTab<double, P>& tabs, int bx,
+                                              int by, int bid, int nblocks);
+
 template <typename T, int P, int TX, int TY, int MODE>
-__global__ void __launch_bounds__(TX* TY)
-    k_sipg_apply(const __grid_constant__ ApplyArgs<T> a, const __grid_constant__ Tab<T, P> tb) {
-  apply_tile<T, P, TX, TY, MODE>(a, tb, blockIdx.x, blockIdx.y, blockIdx.y * gridDim.x + blockIdx.x,
+__device__ __forceinline__ void apply_block(const ApplyArgs<T>& a, const ApplyTab<T, P>& tb, int bx, int by, int bid,
+                                            int nblocks) {
+  if constexpr (sizeof(T) == 8) apply_tile_fx<P, TX, TY, MODE>(a, tb, bx, by, bid, nblocks);
+  else apply_tile<T, P, TX, TY, MODE>(a, tb.t, bx, by, bid, nblocks);
+}
+
+template <typename T, int P, int TX, int TY, int MODE>
+__global__ void __launch_bounds__(TX* TY, apply_min_blocks<T, P, TX, TY>())
+    k_sipg_apply(const __grid_constant__ ApplyArgs<T> a, const __grid_constant__ ApplyTab<T, P> tb) {
+  apply_block<T, P, TX, TY, MODE>(a, tb, blockIdx.x, blockIdx.y, blockIdx.y * gridDim.x + blockIdx.x,
                                  gridDim.x * gridDim.y);
 }
 
@@ -586,9 +645,9 @@ __global__ void __launch_bounds__(TX* TY)
 // (the instances' tiles concatenated; each instance reduces into its own
 // scratch and state, and a converged instance's blocks return at once).
 template <typename T, int P, int TX, int TY, int MODE>
-__global__ void __launch_bounds__(TX* TY)
+__global__ void __launch_bounds__(TX* TY, apply_min_blocks<T, P, TX, TY>())
     k_sipg_apply_batched(const ApplyArgs<T>* __restrict__ insts, const int* __restrict__ tile_start, int ninst,
-                         const __grid_constant__ Tab<T, P> tb) {
+                         const __grid_constant__ ApplyTab<T, P> tb) {
   const int g = blockIdx.x;
   int lo = 0, hi = ninst - 1;
   while (lo < hi) {
@@ -599,73 +658,46 @@ __global__ void __launch_bounds__(TX* TY)
   const ApplyArgs<T> a = insts[lo];
   const int lt = g - __ldg(tile_start + lo);
   const int tiles_x = (a.dim + TX - 1) / TX, tiles_y = (a.dim + TY - 1) / TY;
-  apply_tile<T, P, TX, TY, MODE>(a, tb, lt % tiles_x, lt / tiles_x, lt, tiles_x * tiles_y);
+  apply_block<T, P, TX, TY, MODE>(a, tb, lt % tiles_x, lt / tiles_x, lt, tiles_x * tiles_y);
 }
 
 template <typename T, int P, int TX, int TY>
-cudaError_t launch_apply_tile(int mode, const ApplyArgs<T>& a, const Tab<T, P>& tb, cudaStream_t s) {
-  using S = ApplySmem<T, P, TX, TY>;
+cudaError_t launch_apply_tile(int mode, const ApplyArgs<T>& a, const ApplyTab<T, P>& tb, cudaStream_t s) {
   const int rows = a.nrows > 0 ? a.nrows : a.dim;
   const dim3 grid((a.dim + TX - 1) / TX, (rows + TY - 1) / TY), block(TX, TY);
-  const size_t smem = S::bytes;
-  // the dynamic shared memory opt-in, for all three modes (outside any capture)
-  cudaError_t err = cudaFuncSetAttribute(k_sipg_apply<T, P, TX, TY, APPLY_PLAIN>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(k_sipg_apply<T, P, TX, TY, APPLY_CG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem);
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(k_sipg_apply<T, P, TX, TY, APPLY_RESID>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem);
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(k_sipg_apply<T, P, TX, TY, APPLY_DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem);
+  const size_t smem = apply_smem<T, P, TX, TY>();
+  cudaError_t err = cudaSuccess;
+  bool known = mode == APPLY_PREPARE;
+  if (sizeof(T) == 4) mode = apply_base_mode(mode);  // the FP32 sums are always pivoted
+  // the kernel's dynamic shared memory opt-in (APPLY_PREPARE: of every mode,
+  // before a capture), and its launch
+  auto launch = [&](auto kernel, int kernel_mode) {
+    if (err != cudaSuccess || (mode != APPLY_PREPARE && mode != kernel_mode)) return;
+    known = true;
+    err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess || mode == APPLY_PREPARE) return;
+    kernel<<<grid, block, smem, s>>>(a, tb);
+    count_launch();
+    err = cudaGetLastError();
+  };
+  launch(k_sipg_apply<T, P, TX, TY, APPLY_PLAIN>, APPLY_PLAIN);
+  launch(k_sipg_apply<T, P, TX, TY, APPLY_CG>, APPLY_CG);
+  launch(k_sipg_apply<T, P, TX, TY, APPLY_RESID>, APPLY_RESID);
+  launch(k_sipg_apply<T, P, TX, TY, APPLY_DOT>, APPLY_DOT);
   if constexpr (sizeof(T) == 8) {
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(k_sipg_apply<T, P, TX, TY, APPLY_RESID_PIVOT>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(k_sipg_apply<T, P, TX, TY, APPLY_DOT_PIVOT>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  } else {
-    mode = apply_base_mode(mode);  // the FP32 sums are always pivoted
+    launch(k_sipg_apply<T, P, TX, TY, APPLY_RESID_PIVOT>, APPLY_RESID_PIVOT);
+    launch(k_sipg_apply<T, P, TX, TY, APPLY_DOT_PIVOT>, APPLY_DOT_PIVOT);
   }
-  if (err != cudaSuccess) return err;
-  switch (mode) {
-    case APPLY_PREPARE:
-      return cudaSuccess;
-    case APPLY_PLAIN:
-      k_sipg_apply<T, P, TX, TY, APPLY_PLAIN><<<grid, block, smem, s>>>(a, tb);
-      break;
-    case APPLY_CG:
-      k_sipg_apply<T, P, TX, TY, APPLY_CG><<<grid, block, smem, s>>>(a, tb);
-      break;
-    case APPLY_RESID:
-      k_sipg_apply<T, P, TX, TY, APPLY_RESID><<<grid, block, smem, s>>>(a, tb);
-      break;
-    case APPLY_DOT:
-      k_sipg_apply<T, P, TX, TY, APPLY_DOT><<<grid, block, smem, s>>>(a, tb);
-      break;
-    case APPLY_RESID_PIVOT:
-      if constexpr (sizeof(T) == 8) k_sipg_apply<T, P, TX, TY, APPLY_RESID_PIVOT><<<grid, block, smem, s>>>(a, tb);
-      break;
-    case APPLY_DOT_PIVOT:
-      if constexpr (sizeof(T) == 8) k_sipg_apply<T, P, TX, TY, APPLY_DOT_PIVOT><<<grid, block, smem, s>>>(a, tb);
-      break;
-    default:
-      return cudaErrorInvalidValue;
-  }
-  count_launch();
-  return cudaGetLastError();
+  return known ? err : cudaErrorInvalidValue;
 }
 
 // Tile shapes compiled for each degree: TX = 32 (one warp per element row),
 // TY = 2, 4 or 8 rows; shapes whose shared memory exceeds 227 KB are skipped.
 template <typename T, int P>
 cudaError_t launch_apply_p(const TileCfg& cfg, int mode, const ApplyArgs<T>& a, const HostTables& h, cudaStream_t s) {
-  const Tab<T, P> tb = make_tab<T, P>(h);
+  const ApplyTab<T, P>& tb = apply_tabs<T, P>(h);
   constexpr size_t kMax = 227 * 1024;
-  constexpr bool fits8 = ApplySmem<T, P, 32, 8>::bytes <= kMax;
+  constexpr bool fits8 = apply_smem<T, P, 32, 8>() <= kMax;
   if (cfg.tx != 32 || cfg.tpe != 1) return cudaErrorInvalidValue;
   switch (cfg.ty) {
     case 2:
@@ -679,67 +711,38 @@ cudaError_t launch_apply_p(const TileCfg& cfg, int mode, const ApplyArgs<T>& a, 
   return cudaErrorInvalidValue;
 }
 
+// The modes batched solves use: FP32 the inner CG's DOT, FP64 the served CG and
+// the flexible scheme's steps and residual checks.
 template <typename T, int P, int TX, int TY>
 cudaError_t launch_apply_batched_tile(int mode, const ApplyArgs<T>* insts, const int* tile_start, int ninst,
-                                      int total_tiles, const Tab<T, P>& tb, cudaStream_t s) {
-  const size_t smem = ApplySmem<T, P, TX, TY>::bytes;
-  cudaError_t err = cudaFuncSetAttribute(k_sipg_apply_batched<T, P, TX, TY, APPLY_PLAIN>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(k_sipg_apply_batched<T, P, TX, TY, APPLY_CG>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(k_sipg_apply_batched<T, P, TX, TY, APPLY_RESID>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(k_sipg_apply_batched<T, P, TX, TY, APPLY_DOT>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                      int total_tiles, const ApplyTab<T, P>& tb, cudaStream_t s) {
+  const size_t smem = apply_smem<T, P, TX, TY>();
+  cudaError_t err = cudaSuccess;
+  bool known = mode == APPLY_PREPARE;
+  auto launch = [&](auto kernel, int kernel_mode) {
+    if (err != cudaSuccess || (mode != APPLY_PREPARE && mode != kernel_mode)) return;
+    known = true;
+    err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess || mode == APPLY_PREPARE || total_tiles == 0) return;
+    kernel<<<dim3(total_tiles), dim3(TX, TY), smem, s>>>(insts, tile_start, ninst, tb);
+    count_launch();
+    err = cudaGetLastError();
+  };
   if constexpr (sizeof(T) == 8) {
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(k_sipg_apply_batched<T, P, TX, TY, APPLY_RESID_PIVOT>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(k_sipg_apply_batched<T, P, TX, TY, APPLY_DOT_PIVOT>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  } else {
-    mode = apply_base_mode(mode);
+    launch(k_sipg_apply_batched<T, P, TX, TY, APPLY_CG>, APPLY_CG);
+    launch(k_sipg_apply_batched<T, P, TX, TY, APPLY_RESID_PIVOT>, APPLY_RESID_PIVOT);
+    launch(k_sipg_apply_batched<T, P, TX, TY, APPLY_DOT_PIVOT>, APPLY_DOT_PIVOT);
   }
-  if (err != cudaSuccess || mode == APPLY_PREPARE || total_tiles == 0) return err;
-  const dim3 grid(total_tiles), block(TX, TY);
-  switch (mode) {
-    case APPLY_PLAIN:
-      k_sipg_apply_batched<T, P, TX, TY, APPLY_PLAIN><<<grid, block, smem, s>>>(insts, tile_start, ninst, tb);
-      break;
-    case APPLY_CG:
-      k_sipg_apply_batched<T, P, TX, TY, APPLY_CG><<<grid, block, smem, s>>>(insts, tile_start, ninst, tb);
-      break;
-    case APPLY_RESID:
-      k_sipg_apply_batched<T, P, TX, TY, APPLY_RESID><<<grid, block, smem, s>>>(insts, tile_start, ninst, tb);
-      break;
-    case APPLY_DOT:
-      k_sipg_apply_batched<T, P, TX, TY, APPLY_DOT><<<grid, block, smem, s>>>(insts, tile_start, ninst, tb);
-      break;
-    case APPLY_RESID_PIVOT:
-      if constexpr (sizeof(T) == 8)
-        k_sipg_apply_batched<T, P, TX, TY, APPLY_RESID_PIVOT><<<grid, block, smem, s>>>(insts, tile_start, ninst, tb);
-      break;
-    case APPLY_DOT_PIVOT:
-      if constexpr (sizeof(T) == 8)
-        k_sipg_apply_batched<T, P, TX, TY, APPLY_DOT_PIVOT><<<grid, block, smem, s>>>(insts, tile_start, ninst, tb);
-      break;
-    default:
-      return cudaErrorInvalidValue;
-  }
-  count_launch();
-  return cudaGetLastError();
+  launch(k_sipg_apply_batched<T, P, TX, TY, APPLY_DOT>, APPLY_DOT);
+  return known ? err : cudaErrorInvalidValue;
 }
 
 template <typename T, int P>
 cudaError_t launch_apply_batched_p(const TileCfg& cfg, int mode, const ApplyArgs<T>* insts, const int* tile_start,
                                    int ninst, int total_tiles, const HostTables& h, cudaStream_t s) {
-  const Tab<T, P> tb = make_tab<T, P>(h);
+  const ApplyTab<T, P>& tb = apply_tabs<T, P>(h);
   constexpr size_t kMax = 227 * 1024;
-  constexpr bool fits8 = ApplySmem<T, P, 32, 8>::bytes <= kMax;
+  constexpr bool fits8 = apply_smem<T, P, 32, 8>() <= kMax;
   // batched solves keep 32-element rows: their tiles are laid out by
   // tile_start for that width
   if (cfg.tx != 32) return cudaErrorInvalidValue;
@@ -754,12 +757,6 @@ cudaError_t launch_apply_batched_p(const TileCfg& cfg, int mode, const ApplyArgs
                                                                   s);
   }
   return cudaErrorInvalidValue;
-}
-
-template <typename T>
-inline size_t apply_smem_bytes(int p, int ty) {
-  size_t n1 = p + 1, te = 32 * ty;
-  return (n1 * n1 * te + ty * 2 * n1 * 33 + (ty + 1) * 2 * n1 * 32) * sizeof(T);
 }
 
 }  // namespace sipg

@@ -10,35 +10,32 @@
 // Here a CTA holds EX x EY elements and gives each output node its own thread:
 // the same operations spread over (p+1)^2 times more warps, on more SMs.
 //
-// Each output is formed by exactly the operations, in exactly the order, of
-// the element-per-thread kernel's column form (the FP64 form): one chain
-// from the face nodes' +-Q and the x-face lifting through the weighted volume
-// sums sum_i w_j K(i1,i) u(i,j) and sum_i w_i1 K(j,i) u(i1,i) to the y-face
-// lifting.  Face
-// values (J, Q) come from the same one-sided traces and derivatives combined
-// by the same expression.  So the result is bit-identical to every other
-// FP64 tile shape; only the CG reductions (p.Ap, r.r) group their partial
-// sums differently.
+// The sums are the fixed-point ones of sipg_apply_fx.cuh (sipg_fx.cuh): the
+// same integers, whose sums do not depend on their order, so the result is
+// bit-identical to every other FP64 tile shape; only the CG reductions (p.Ap,
+// r.r) group their partial sums differently.
 //
 // A CTA works through tiles blockIdx.x, blockIdx.x + gridDim.x, ... with the
 // grid at most the resident CTAs, so a mesh of any size has at most a few
-// thousand reduction partials.  Phases per tile (static shared memory, a few
-// KB):
-//   0  the tables, and the nodal blocks of the EX x EY elements and of the
-//      2 (EX + EY) halo elements around them (from L2: small meshes live
-//      there), with p = r + beta p_old formed on the fly in the CG mode;
-//   1  one thread per face node: trace and normal derivative of each side,
-//      combined into J and Q (both sides present inside the mesh, one side on
-//      the domain boundary);
-//   2  one thread per output node, then the epilogue (store, direction store
-//      in the CG mode, deterministic grid reduction in the CG / DOT /
-//      residual modes).
+// thousand reduction partials.  Phases per tile (static shared memory, tens of
+// KB at most):
+//   0  the values of the EX x EY elements and of the 2 (EX + EY) halo elements
+//      around them (from L2: small meshes live there), with p = r + beta p_old
+//      formed on the fly in the CG mode, and the elements' scales;
+//   1  their parity form, four mirrored nodes per thread;
+//   2  w times the normal derivatives, one face component per thread;
+//   3  J and Q, one face component per thread;
+//   4  one parity component of the output per thread;
+//   5  one output node per thread, then the epilogue (store, direction store
+//      in the CG mode, deterministic grid reduction in the CG / DOT / residual
+//      modes).
+// A tile with values out of the fixed-point range takes the plain FP64 code.
 #pragma once
 
 #include <algorithm>
 #include <atomic>
 
-#include "sipg_apply.cuh"
+#include "sipg_apply_fx.cuh"
 
 namespace sipg {
 
@@ -52,163 +49,264 @@ struct PernodeShape {
   static constexpr int NY = EX * (EY + 1) * N1;        // y-face nodes: [EY+1][EX][N1]
 };
 
-// The CTA's shared memory: the nodal blocks of its tile and halo ring, the
-// face values, and the tables.
-template <typename T, int P, int SHAPE>
-struct PernodeSmem {
+// The CTA's shared memory.
+template <int P, int SHAPE>
+struct PernodeFxSmem {
   using S = PernodeShape<P, SHAPE>;
-  T us[S::SX * S::SY * S::NN];  // slot (sy, sx) = element (y0 - 1 + sy, x0 - 1 + sx), values [i1 * N1 + i2]
-  T xj[S::NX], xq[S::NX], yj[S::NY], yq[S::NY];
-  T tw[S::N1], twh[S::N1], td0[S::N1], tdn[S::N1], tkw[S::NN * S::N1];
+  static constexpr int NSLOT = S::SX * S::SY;
+  int2 us[NSLOT * S::NN];     // slot (sy, sx) = element (y0 - 1 + sy, x0 - 1 + sx): values, then parity form
+  double own[S::NE * S::NN];  // the tile's values [node][element]
+  static constexpr int RX = S::EY * S::SX * S::N1, RY = S::SY * S::EX * S::N1;
+  long long r0[RX + RY], rN[RX + RY];  // derivatives of the x faces, then the y faces: 0 side, N side
+  long long xj[S::NX], xq[S::NX], yj[S::NY], yq[S::NY];
+  long long tot[S::NE * S::NN];  // the output's parity components
+  unsigned mag[NSLOT];           // zero between tiles
+  int be[NSLOT], bo[S::NE];      // scales of the slots' values, of the outputs
+  int xbe[S::EY * (S::EX + 1)], ybe[S::EX * (S::EY + 1)];  // of the faces
+  FxTab<P> fx;
+  int2 nu[FxTab<P>::NE];
+  double wnu[FxTab<P>::NE];
+  bool large;
 };
 
-// The tables into shared memory (indexed per thread below: a constant-bank
-// read whose address differs across the warp would serialise).  The caller
-// synchronises before their first use.
-template <typename T, int P, int SHAPE>
-__device__ __forceinline__ void pernode_tables(PernodeSmem<T, P, SHAPE>& sm, const Tab<T, P>& tb) {
-  using S = PernodeShape<P, SHAPE>;
+// The fixed-point tables into shared memory (indexed per thread below: a
+// constant-bank read whose address differs across the warp would serialise),
+// the penalty's coefficients, and cleared magnitudes.
+template <int P, int SHAPE>
+__device__ __forceinline__ void pernode_fx_tables(PernodeFxSmem<P, SHAPE>& sm, const FxTab<P>& fx, double nu) {
   const int t = threadIdx.x;
-  for (int k = t; k < S::NN * S::N1; k += S::NT) sm.tkw[k] = tb.KW[k];
-  if (t < S::N1) {
-    sm.tw[t] = tb.w[t];
-    sm.twh[t] = tb.WH[t];
-    sm.td0[t] = tb.D0[t];
-    sm.tdn[t] = tb.DN[t];
+  static_assert(sizeof(FxTab<P>) % 8 == 0, "copied as 8-byte words");
+  for (int k = t; k < (int)(sizeof(FxTab<P>) / 8); k += PernodeShape<P, SHAPE>::NT)
+    reinterpret_cast<long long*>(&sm.fx)[k] = reinterpret_cast<const long long*>(&fx)[k];
+  for (int k = t; k < PernodeFxSmem<P, SHAPE>::NSLOT; k += PernodeShape<P, SHAPE>::NT) sm.mag[k] = 0;
+  const bool large = fx_large_nu(nu * fx.wmax, fx.sk);
+  if (t < FxTab<P>::NE) {
+    sm.wnu[t] = fx.w[t] * nu;
+    sm.nu[t] = large ? make_int2(0, 0) : fx_nu(fx.w[t] * nu, fx.sk);
   }
+  if (t == 0) sm.large = large;
+  __syncthreads();
 }
 
-// One tile (origin x0, y0): phases 0-2, returning this thread's share of the
+// One tile (origin x0, y0): phases 0-5, returning this thread's share of the
 // reduction (p.Ap in the CG / DOT modes, r.r in the residual mode).
 // kCoherent: read a.in and pold through L2 only -- for a caller that runs
 // while other CTAs of the same grid write them (the persistent CG).
-template <typename T, int P, int SHAPE, int MODE, bool kCoherent>
-__device__ __forceinline__ T pernode_tile(const ApplyArgs<T>& a, PernodeSmem<T, P, SHAPE>& sm, int x0, int y0,
-                                          bool first, T beta, const T* __restrict__ pold, T* __restrict__ pnew) {
+template <int P, int SHAPE, int MODE, bool kCoherent>
+__device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, PernodeFxSmem<P, SHAPE>& sm,
+                                                  const ApplyTab<double, P>& tabs, int x0, int y0, bool first,
+                                                  double beta, const double* __restrict__ pold,
+                                                  double* __restrict__ pnew) {
   using S = PernodeShape<P, SHAPE>;
-  constexpr int N = P, N1 = S::N1, NN = S::NN, EX = S::EX, NE = S::NE, NT = S::NT;
+  using Tb = FxTab<P>;
+  constexpr int N = P, N1 = S::N1, NN = S::NN, EX = S::EX, EY = S::EY, NE = S::NE, NT = S::NT;
   constexpr int SX = S::SX, SY = S::SY, NX = S::NX, NY = S::NY, NSLOT = SX * SY;
+  constexpr int HE = Tb::NE, HO = Tb::NO;
   constexpr bool kDot = (MODE == APPLY_CG || MODE == APPLY_DOT);
-  T* __restrict__ us = sm.us;
-  T* __restrict__ xj = sm.xj;
-  T* __restrict__ xq = sm.xq;
-  T* __restrict__ yj = sm.yj;
-  T* __restrict__ yq = sm.yq;
-  const T* __restrict__ tw = sm.tw;
-  const T* __restrict__ twh = sm.twh;
-  const T* __restrict__ td0 = sm.td0;
-  const T* __restrict__ tdn = sm.tdn;
-  const T* __restrict__ tkw = sm.tkw;
+  const FxTab<P>& fx = sm.fx;
   const int t = threadIdx.x;
   const int dim = a.dim;
   const size_t noe = (size_t)dim * dim;
-  const T nu = a.nu;
-  auto ldin = [&](const T* p) -> T { return kCoherent ? __ldcg(p) : __ldg(p); };
-  T acc = T(0);
-  // ---- phase 0: nodal blocks ------------------------------------------------
+  auto ldin = [&](const double* p) -> double { return kCoherent ? __ldcg(p) : __ldg(p); };
+  auto corner = [](int sx, int sy) { return (sx == 0 || sx == SX - 1) && (sy == 0 || sy == SY - 1); };
+  auto in_mesh = [&](int sx, int sy) {
+    const int gx = x0 - 1 + sx, gy = y0 - 1 + sy;
+    return gx >= 0 && gx < dim && gy >= 0 && gy < dim;
+  };
+  // ---- phase 0: values and magnitudes ----------------------------------------
   for (int idx = t; idx < NSLOT * NN; idx += NT) {
     const int k = idx / NSLOT, sl = idx - k * NSLOT;
     const int sy = sl / SX, sx = sl - sy * SX;
-    const int gx = x0 - 1 + sx, gy = y0 - 1 + sy;
-    const bool corner = (sx == 0 || sx == SX - 1) && (sy == 0 || sy == SY - 1);
-    T v = T(0);
-    if (!corner && gx >= 0 && gx < dim && gy >= 0 && gy < dim) {
-      const size_t gk = (size_t)k * noe + (size_t)gy * dim + gx;
+    double v = 0.0;
+    if (!corner(sx, sy) && in_mesh(sx, sy)) {
+      const size_t gk = (size_t)k * noe + (size_t)(y0 - 1 + sy) * dim + (x0 - 1 + sx);
       v = ldin(a.in + gk);
       if (MODE == APPLY_CG && !first) v = fma(beta, ldin(pold + gk), v);
+      atomicMax(&sm.mag[sl], fx_mag(v));
     }
-    us[sl * NN + k] = v;
+    sm.us[sl * NN + k] = make_int2(__double2loint(v), __double2hiint(v));
+    if (sx > 0 && sx < SX - 1 && sy > 0 && sy < SY - 1) sm.own[k * NE + (sy - 1) * EX + sx - 1] = v;
   }
   __syncthreads();
-
-  // ---- phase 1: J and Q of every face node of the tile -----------------------
+  // ---- phase 1: parity form ---------------------------------------------------
+  bool bad = fx_biased(a.nu) > kFxMaxNu;
+  for (int sl = t; sl < NSLOT; sl += NT) {
+    const unsigned b = sm.mag[sl] >> 21;
+    bad = bad || b >= (unsigned)kFxMaxExp;
+    if (b < (unsigned)kFxMinExp && b > 0) bad = true;  // (b = 0: zeros and denormals, told apart below)
+    sm.be[sl] = fx_be(sm.mag[sl]);
+  }
+  for (int task = t; task < NSLOT * HE * HE; task += NT) {
+    const int sl = task / (HE * HE), q2 = task - sl * (HE * HE), i = q2 / HE, j = q2 - i * HE;
+    const int be = fx_be(sm.mag[sl]);
+    const bool mi = 2 * i == N, mj = 2 * j == N;
+    int2* u = sm.us + sl * NN;
+    const int k0 = i * N1 + j, k1 = (N - i) * N1 + j, k2 = i * N1 + N - j, k3 = (N - i) * N1 + N - j;
+    auto raw = [&](int k) {
+      const double v = __hiloint2double(u[k].y, u[k].x);
+      bad = bad || (fx_biased(v) == 0 && v != 0.0 && be == kFxMinExp);
+      return v;
+    };
+    long long q[4];
+    q[0] = fx_fix(raw(k0), be);
+    q[1] = mi ? 0 : fx_fix(raw(k1), be);
+    q[2] = mj ? 0 : fx_fix(raw(k2), be);
+    q[3] = mi || mj ? 0 : fx_fix(raw(k3), be);
+    fx_quad(q);
+    u[k0] = fx_limbs_of(q[0]);
+    if (!mi) u[k1] = fx_limbs_of(q[1]);
+    if (!mj) u[k2] = fx_limbs_of(q[2]);
+    if (!mi && !mj) u[k3] = fx_limbs_of(q[3]);
+  }
+  if (__syncthreads_or(bad)) {  // out of the fixed-point range: the plain code, one element per thread
+    double r = 0.0;
+    auto ld = [&](int k, size_t e) -> double {
+      const double v = ldin(a.in + (size_t)k * noe + e);
+      return MODE == APPLY_CG && !first ? fma(beta, ldin(pold + (size_t)k * noe + e), v) : v;
+    };
+    if (t < NE && x0 + t % EX < dim && y0 + t / EX < dim)
+      r = plain_element<P, MODE>(a, tabs.t, x0 + t % EX, y0 + t / EX, ld, pnew);
+    for (int sl = t; sl < NSLOT; sl += NT) sm.mag[sl] = 0;
+    __syncthreads();
+    return r;
+  }
+  // ---- phase 2: normal derivatives -------------------------------------------
+  constexpr int TX_ = EY * SX * N1, TY_ = SY * EX * N1;
+  for (int task = t; task < TX_ + TY_; task += NT) {
+    const bool x = task < TX_;
+    const int q = x ? task : task - TX_;
+    const int b = q % N1, r = q / N1, wb = b < HE ? b : N - b;
+    // x: tile row r / SX, slot column r % SX; y: slot row r / EX, tile column r % EX
+    const int sl = x ? (r / SX + 1) * SX + r % SX : (r / EX) * SX + r % EX + 1;
+    const int2* u = sm.us + sl * NN;
+    long long r0, rN;
+    fx_derivatives<P>(fx, wb, [&](int k, bool odd) {
+      const int kk = odd ? N - k : k;
+      return x ? u[kk * N1 + b] : u[b * N1 + kk];
+    }, r0, rN);
+    sm.r0[task] = r0;
+    sm.rN[task] = rN;
+  }
+  for (int sl = t; sl < NSLOT; sl += NT) sm.mag[sl] = 0;  // for the next tile
+  __syncthreads();
+  // ---- phase 3: J and Q ---------------------------------------------------------
   for (int f = t; f < NX + NY; f += NT) {
-    T u0 = T(0), d0 = T(0), uN = T(0), dN = T(0);
-    bool zv, nv;  // 0-side / N-side element inside the mesh
-    int j;
-    if (f < NX) {
-      // x face fx of tile row ey: the left element (slot fx) is its N-side
-      // (i1 = P), the right element (slot fx + 1) its 0-side (i1 = 0)
-      j = f % N1;
-      const int r = f / N1, fx = r % (EX + 1), ey = r / (EX + 1);
-      const int gy = y0 + ey, gxl = x0 + fx - 1;
-      nv = gy < dim && gxl >= 0 && gxl < dim;
-      zv = gy < dim && gxl + 1 < dim;
-      const T* L = us + ((ey + 1) * SX + fx) * NN;
-      const T* R = L + NN;
-      if (zv) {
-        u0 = R[j];
-#pragma unroll
-        for (int i = 0; i < N1; ++i) d0 = fma(td0[i], R[i * N1 + j], d0);
-      }
-      if (nv) {
-        uN = L[N * N1 + j];
-#pragma unroll
-        for (int i = 0; i < N1; ++i) dN = fma(tdn[i], L[i * N1 + j], dN);
-      }
-    } else {
-      // y face fy of tile column ex: the upper element (slot row fy) is its
-      // 0-side (i2 = 0), the lower element (slot row fy + 1) its N-side (i2 = P)
-      const int g = f - NX;
-      j = g % N1;
-      const int r = g / N1, ex = r % EX, fy = r / EX;
-      const int gx = x0 + ex, gyu = y0 + fy - 1;
-      zv = gx < dim && gyu >= 0 && gyu < dim;
-      nv = gx < dim && gyu + 1 < dim;
-      const T* Up = us + (fy * SX + ex + 1) * NN;
-      const T* Dn = Up + SX * NN;
-      if (zv) {
-        u0 = Up[j * N1];
-#pragma unroll
-        for (int i = 0; i < N1; ++i) d0 = fma(td0[i], Up[j * N1 + i], d0);
-      }
-      if (nv) {
-        uN = Dn[j * N1 + N];
-#pragma unroll
-        for (int i = 0; i < N1; ++i) dN = fma(tdn[i], Dn[j * N1 + i], dN);
-      }
+    const bool x = f < NX;
+    const int q = x ? f : f - NX, b = q % N1, r = q / N1, wb = b < HE ? b : N - b;
+    int s0, sN, i0, iN, face;  // slots of the two sides, their derivatives
+    bool zv, nv;
+    if (x) {  // x face c of tile row ey: the left slot is the N side, the right one the 0 side
+      const int c = r % (EX + 1), ey = r / (EX + 1);
+      sN = (ey + 1) * SX + c, s0 = sN + 1;
+      iN = (ey * SX + c) * N1 + b, i0 = iN + N1;
+      nv = in_mesh(c, ey + 1), zv = in_mesh(c + 1, ey + 1);
+      face = ey * (EX + 1) + c;
+    } else {  // y face c of tile column ex: the upper slot is the 0 side, the lower one the N side
+      const int ex = r % EX, c = r / EX;
+      s0 = c * SX + ex + 1, sN = s0 + SX;
+      i0 = TX_ + (c * EX + ex) * N1 + b, iN = i0 + EX * N1;
+      zv = in_mesh(ex + 1, c), nv = in_mesh(ex + 1, c + 1);
+      face = c * EX + ex;
     }
-    T J, Q;
-    face_combine<T>(tw[j], twh[j], nu, zv && nv, u0, d0, uN, dN, J, Q);
-    if (f < NX) {
-      xj[f] = J;
-      xq[f] = Q;
+    if (!zv && !nv) continue;
+    const int2 *u0 = sm.us + s0 * NN, *uN = sm.us + sN * NN;
+    const int ke = x ? b : b * N1, ko = x ? N * N1 + b : b * N1 + N;
+    const int be0 = sm.be[s0], beN = sm.be[sN];
+    long long J, Q;
+    fx_face<false>(sm.large, sm.wnu[wb], sm.nu[wb], fx.sk, zv, nv, fx_trace0(u0[ke], u0[ko]),
+                   sm.r0[i0], be0, fx_traceN(uN[ke], uN[ko]), sm.rN[iN], beN, 0.0, 0, J, Q);
+    const int bf = !zv ? beN : (!nv ? be0 : max(be0, beN));
+    if (x) {
+      sm.xj[q] = J;
+      sm.xq[q] = Q;
+      if (b == 0) sm.xbe[face] = bf;
     } else {
-      yj[f - NX] = J;
-      yq[f - NX] = Q;
+      sm.yj[q] = J;
+      sm.yq[q] = Q;
+      if (b == 0) sm.ybe[face] = bf;
     }
   }
   __syncthreads();
-
-  // ---- phase 2: one output node per thread ------------------------------------
+  // ---- phase 4: the output's parity components -----------------------------------
+  if (t < NE * NN) {
+    const int le = t % NE, k = t / NE, ex = le % EX, ey = le / EX;
+    const int ka = k / N1, kb = k - ka * N1;  // slot indices along x and y
+    if (x0 + ex < dim && y0 + ey < dim) {
+      const int sl = (ey + 1) * SX + ex + 1;
+      const int2* u = sm.us + sl * NN;
+      const int bs = sm.be[sl];
+      const int fL = ey * (EX + 1) + ex, fR = fL + 1, fU = ey * EX + ex, fD = fU + EX;  // faces
+      const int bL = sm.xbe[fL], bR = sm.xbe[fR], bU = sm.ybe[fU], bD = sm.ybe[fD];
+      int be = max(bs, max(max(bL, bR), max(bD, bU)) - kFxRoom);
+      if (sm.large) {
+        unsigned m = 0;
+        for (int b = 0; b < N1; ++b) {
+          m = max(m, max(fx_mag(__longlong_as_double(sm.xq[fL * N1 + b])), fx_mag(__longlong_as_double(sm.xq[fR * N1 + b]))));
+          m = max(m, max(fx_mag(__longlong_as_double(sm.yq[fD * N1 + b])), fx_mag(__longlong_as_double(sm.yq[fU * N1 + b]))));
+        }
+        be += max(0, fx_raise(be, fx.sk, m));
+      }
+      const int so = be - bs, xp = fx_exp(be, fx.sk);
+      auto own = [&](int kk) { return so > 0 ? fx_shift(u[kk], min(so, 63)) : u[kk]; };
+      const bool oa = ka >= HE, ob = kb >= HE;  // odd indices sit at the mirrored slots
+      const int ia = oa ? N - ka : ka, ib = ob ? N - kb : kb;
+      FxAcc s = fx_zero();
+      // x sums and lift, then y
+      const int na = oa ? HO : HE, nb = ob ? HO : HE;
+      const int2 *ta = oa ? fx.ko + ia * HO * HE + ib : fx.ke + ia * HE * HE + ib;
+      const int2 *tb = ob ? fx.ko + ib * HO * HE + ia : fx.ke + ib * HE * HE + ia;
+#pragma unroll
+      for (int q = 0; q < HE; ++q)
+        if (q < na) fx_mac(s, ta[q * HE], own((oa ? N - q : q) * N1 + kb));
+#pragma unroll
+      for (int q = 0; q < HE; ++q)
+        if (q < nb) fx_mac(s, tb[q * HE], own(ka * N1 + (ob ? N - q : q)));
+      const long long jl = fx_scaled(sm.xj[fL * N1 + kb], be - bL), jr = fx_scaled(sm.xj[fR * N1 + kb], be - bR);
+      const long long jd = fx_scaled(sm.yj[fD * N1 + ka], be - bD), ju = fx_scaled(sm.yj[fU * N1 + ka], be - bU);
+      fx_mac(s, (oa ? fx.lo : fx.le)[ia * HE + ib], fx_limbs_of(oa ? jl + jr : jl - jr));
+      fx_mac(s, (ob ? fx.lo : fx.le)[ib * HE + ia], fx_limbs_of(ob ? jd + ju : jd - ju));
+      long long r = fx_total(s);
+      auto half_q = [&](long long q, int bf) {
+        return sm.large ? fx_units(__longlong_as_double(q), xp) : fx_scaled(q, be - bf);
+      };
+      if (ia == 0) {
+        const long long ql = half_q(sm.xq[fL * N1 + kb], bL), qr = half_q(sm.xq[fR * N1 + kb], bR);
+        r += oa ? ql + qr : ql - qr;
+      }
+      if (ib == 0) {
+        const long long qd = half_q(sm.yq[fD * N1 + ka], bD), qu = half_q(sm.yq[fU * N1 + ka], bU);
+        r += ob ? qd + qu : qd - qu;
+      }
+      sm.tot[le * NN + k] = r;
+      if (k == 0) sm.bo[le] = xp;
+    }
+  }
+  __syncthreads();
+  // ---- phase 5: one output node per thread ---------------------------------------
+  double acc = 0.0;
   if (t < NE * NN) {
     const int le = t % NE, k = t / NE;  // element fastest: neighbouring threads store neighbouring elements
-    const int ex = le % EX, ey = le / EX;
-    const int i1 = k / N1, j = k - i1 * N1;
+    const int ex = le % EX, ey = le / EX, i1 = k / N1, j = k - i1 * N1;
     const int gx = x0 + ex, gy = y0 + ey;
     if (gx < dim && gy < dim) {
-      const T* E = us + ((ey + 1) * SX + ex + 1) * NN;
-      const int fl = (ey * (EX + 1) + ex) * N1;  // left x face; the right one is fl + N1
-      const int fd = ((ey + 1) * EX + ex) * N1;  // down y face; the up one is fd - EX * N1
-      const int fu = fd - EX * N1;
-      const bool xf = (i1 == 0) || (i1 == N);
-      const T seed = face_seed<T, N>(i1, j, xf ? xq[fl + j] : T(0), xf ? xq[fl + N1 + j] : T(0),
-                                     (j == 0) ? yq[fd + i1] : T(0), (j == N) ? yq[fu + i1] : T(0));
-      T v = fma(td0[i1], xj[fl + j], fma(tdn[i1], xj[fl + N1 + j], seed));
-#pragma unroll
-      for (int i = 0; i < N1; ++i) v = fma(tkw[(i1 * N1 + i) * N1 + j], E[i * N1 + j], v);
-#pragma unroll
-      for (int i = 0; i < N1; ++i) v = fma(tkw[(j * N1 + i) * N1 + i1], E[i1 * N1 + i], v);
-      v = fma(td0[j], yj[fd + i1], v);
-      v = fma(tdn[j], yj[fu + i1], v);
+      const long long* T = sm.tot + le * NN;
+      const int i = i1 < N - i1 ? i1 : N - i1, jj = j < N - j ? j : N - j;
+      auto row = [&](int ka) -> long long {  // the component at y node j
+        if (2 * jj == N) return T[ka * N1 + jj];
+        const long long ev = T[ka * N1 + jj], od = T[ka * N1 + N - jj];
+        return j == jj ? ev + od : ev - od;
+      };
+      long long r = row(i);
+      if (2 * i != N) r = i1 == i ? r + row(N - i) : r - row(N - i);
+      const double v = fx_double(r, sm.bo[le]);
       const size_t gk = (size_t)k * noe + (size_t)gy * dim + gx;
       if (MODE == APPLY_RESID) {
-        const T rv = __ldg(a.b + gk) - v;
+        const double rv = __ldg(a.b + gk) - v;
         a.out[gk] = rv;
         acc = fma(rv, rv, acc);
       } else {
         a.out[gk] = v;
-        const T c = E[k];
+        const double c = sm.own[k * NE + le];
         if (MODE == APPLY_CG) pnew[gk] = c;
         if (kDot) acc = fma(c, v, acc);
       }
@@ -220,10 +318,10 @@ __device__ __forceinline__ T pernode_tile(const ApplyArgs<T>& a, PernodeSmem<T, 
 
 template <typename T, int P, int SHAPE, int MODE>
 __global__ void __launch_bounds__(PernodeShape<P, SHAPE>::NT)
-    k_sipg_apply_pernode(const __grid_constant__ ApplyArgs<T> a, const __grid_constant__ Tab<T, P> tb) {
+    k_sipg_apply_pernode(const __grid_constant__ ApplyArgs<T> a, const __grid_constant__ ApplyTab<T, P> tb) {
   using S = PernodeShape<P, SHAPE>;
   constexpr int EX = S::EX, EY = S::EY, NT = S::NT;
-  __shared__ PernodeSmem<T, P, SHAPE> sm;
+  __shared__ PernodeFxSmem<P, SHAPE> sm;
   __shared__ T red_sh[32];
 
   constexpr bool kDot = (MODE == APPLY_CG || MODE == APPLY_DOT);
@@ -245,13 +343,13 @@ __global__ void __launch_bounds__(PernodeShape<P, SHAPE>::NT)
   }
   const T* __restrict__ pold = par ? a.pbuf1 : a.pbuf0;
   T* __restrict__ pnew = par ? a.pbuf0 : a.pbuf1;
-  pernode_tables<T, P, SHAPE>(sm, tb);
+  pernode_fx_tables<P, SHAPE>(sm, tb.fx, a.nu);
   T acc = T(0);
   // the CTA's tiles: blockIdx.x, + gridDim.x, ... (the grid is at most the
   // resident CTAs, so the reduction has few partials on any mesh)
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int x0 = (tile % tiles_x) * EX, y0 = a.row0 + (tile / tiles_x) * EY;
-    acc += pernode_tile<T, P, SHAPE, MODE, false>(a, sm, x0, y0, first, beta, pold, pnew);
+    acc += pernode_tile_fx<P, SHAPE, MODE, false>(a, sm, tb, x0, y0, first, beta, pold, pnew);
   }
 
   if (MODE != APPLY_PLAIN) {
@@ -282,7 +380,7 @@ int pernode_resident_blocks(K kernel, int threads) {
 }
 
 template <typename T, int P, int SHAPE>
-cudaError_t launch_apply_pernode_shape(int mode, const ApplyArgs<T>& a, const Tab<T, P>& tb, cudaStream_t s) {
+cudaError_t launch_apply_pernode_shape(int mode, const ApplyArgs<T>& a, const ApplyTab<T, P>& tb, cudaStream_t s) {
   using S = PernodeShape<P, SHAPE>;
   if (mode == APPLY_PREPARE) return cudaSuccess;  // static shared memory: no attribute to set
   const int rows = a.nrows > 0 ? a.nrows : a.dim;
@@ -329,7 +427,7 @@ template <typename T, int P>
 cudaError_t launch_apply_pernode(const TileCfg& cfg, int mode, const ApplyArgs<T>& a, const HostTables& h,
                                  cudaStream_t s) {
   if (cfg.ty != pernode_ey(P)) return cudaErrorInvalidConfiguration;
-  const Tab<T, P> tb = make_tab<T, P>(h);
+  const ApplyTab<T, P>& tb = apply_tabs<T, P>(h);
   if (cfg.tx == pernode_ex(P, 0)) return launch_apply_pernode_shape<T, P, 0>(mode, a, tb, s);
   if (cfg.tx == pernode_ex(P, 1)) return launch_apply_pernode_shape<T, P, 1>(mode, a, tb, s);
   return cudaErrorInvalidConfiguration;
