@@ -162,6 +162,110 @@ __global__ void k_rhs(double* __restrict__ b, int p, int dim, double pen, const 
   }
 }
 
+// ---- right-hand sides of sine products (SIPG_SOL_SINSIN, SIPG_SOL_MODES) ----
+//
+// f = sum_q F_q sin(k_q x) sin(l_q y) on a tensor mesh: the sines depend on one
+// axis each, so they are tabulated per axis node -- 2 NM dim (p + 1) of them
+// instead of 2 NM per DoF -- and a DoF costs NM FP64 multiply-adds and the
+// quadrature weight.  k_rhs spent 8 FP64 sines on each DoF of a 4-mode f:
+// 512^2, p = 6: 5846 us; here 235 us, of which the FP64 pipe needs 110 for its
+// NM + 1 operations per DoF.
+struct SineModes {
+  int n;
+  double F[8], U[8], k[8], l[8];  // f = sum F s s, u = sum U s s
+};
+
+static SineModes sine_modes(const ProblemArgs& pa) {
+  SineModes m;
+  std::memset(&m, 0, sizeof(m));
+  if (pa.sol == SIPG_SOL_SINSIN) {
+    const double tp = 2 * M_PI;
+    m.n = 1;
+    m.F[0] = 2 * tp * tp;
+    m.U[0] = 1.0;
+    m.k[0] = m.l[0] = tp;
+  } else {
+    m.n = pa.modes.nmodes;
+    for (int q = 0; q < m.n; ++q) {
+      m.k[q] = pa.modes.k[q] * M_PI;
+      m.l[q] = pa.modes.l[q] * M_PI;
+      m.F[q] = pa.modes.amp[q];
+      m.U[q] = pa.modes.amp[q] / (m.k[q] * m.k[q] + m.l[q] * m.l[q]);
+    }
+  }
+  return m;
+}
+
+// sx[(q n + i) dim + col] = sin(k_q x), sy[(q n + i) dim + row] = sin(l_q y) for
+// q < nm (zero beyond the problem's modes); blockIdx.y = q n + i.
+__global__ void k_sine_tables(double* __restrict__ sx, double* __restrict__ sy, int n, int dim,
+                              const __grid_constant__ SineModes m, const __grid_constant__ RhsTables tb,
+                              const double* __restrict__ xcol, const double* __restrict__ yrow) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= dim) return;
+  const int q = blockIdx.y / n, i = blockIdx.y % n;
+  const size_t at = (size_t)blockIdx.y * dim + c;
+  sx[at] = q < m.n ? sin(m.k[q] * (xcol[c] + tb.nodes[i])) : 0.0;
+  sy[at] = q < m.n ? sin(m.l[q] * (yrow[c] + tb.nodes[i])) : 0.0;
+}
+
+// One thread per element, NM the table's modes; the boundary terms in k_rhs's
+// order.
+template <int NM>
+__global__ void __launch_bounds__(128)
+    k_rhs_sines(double* __restrict__ b, int p, int dim, double pen, const __grid_constant__ SineModes m,
+                const __grid_constant__ RhsTables tb, const double* __restrict__ sx, const double* __restrict__ sy) {
+  const unsigned noe = (unsigned)dim * (unsigned)dim;
+  const unsigned e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= noe) return;
+  const int n = p + 1, N = p;
+  const int row = (int)(e / (unsigned)dim), col = (int)(e % (unsigned)dim);
+  auto B = [&](int i1, int i2) -> double& { return b[((size_t)i1 * n + i2) * noe + e]; };
+  auto X = [&](int q, int i) { return __ldg(sx + (size_t)(q * n + i) * dim + col); };
+  auto Y = [&](int q, int i) { return __ldg(sy + (size_t)(q * n + i) * dim + row); };
+  for (int i1 = 0; i1 < n; ++i1) {
+    double c[NM];
+#pragma unroll
+    for (int q = 0; q < NM; ++q) c[q] = q < m.n ? m.F[q] * X(q, i1) : 0.0;
+#pragma unroll 3
+    for (int i2 = 0; i2 < n; ++i2) {
+      double f = 0.0;
+#pragma unroll
+      for (int q = 0; q < NM; ++q) f = fma(c[q], Y(q, i2), f);
+      B(i1, i2) = tb.w[i1] * tb.w[i2] * f;
+    }
+  }
+  const bool isD = row == dim - 1, isU = row == 0, isL = col == 0, isR = col == dim - 1;
+  if (!(isD || isU || isL || isR)) return;
+  auto u = [&](int i1, int i2) {
+    double v = 0.0;
+#pragma unroll
+    for (int q = 0; q < NM; ++q)
+      if (q < m.n) v = fma(m.U[q] * X(q, i1), Y(q, i2), v);
+    return v;
+  };
+  // an element's faces by strip position: DOWN and UP at col, LEFT and RIGHT at row
+  const int strips[2] = {min(row, col), max(row, col)};
+  for (int q = 0; q < (row == col ? 1 : 2); ++q) {
+    const int xx = strips[q];
+    const bool D = isD && col == xx, U = isU && col == xx, L = isL && row == xx, R = isR && row == xx;
+    if (!(D || U || L || R)) continue;
+    for (int i = 0; i <= N; ++i) {
+      const double gD = D ? u(i, 0) : 0.0, gU = U ? u(i, N) : 0.0, gL = L ? u(0, i) : 0.0, gR = R ? u(N, i) : 0.0;
+      if (D) B(i, 0) += pen * tb.weights[i] * gD;
+      if (U) B(i, N) += pen * tb.weights[i] * gU;
+      if (L) B(0, i) += pen * tb.weights[i] * gL;
+      if (R) B(N, i) += pen * tb.weights[i] * gR;
+      for (int j = 0; j <= N; ++j) {
+        if (D) B(i, j) -= -1 * tb.weights[i] * tb.D[j * n + 0] * gD;
+        if (U) B(i, j) -= tb.weights[i] * tb.D[j * n + N] * gU;
+        if (L) B(j, i) -= -1 * tb.weights[i] * tb.D[j * n + 0] * gL;
+        if (R) B(j, i) -= tb.weights[i] * tb.D[j * n + N] * gR;
+      }
+    }
+  }
+}
+
 constexpr int kErrThreads = 128;
 
 __global__ void __launch_bounds__(kErrThreads)
@@ -276,20 +380,51 @@ __global__ void k_mesh_axes(double* __restrict__ xcol, double* __restrict__ yrow
 // queued behind other work on s, or beside other streams' work, waits for
 // nothing.
 sipg_status rhs_f64(const sipg_op* op, int sol, const sipg_modes* modes, double* d_b, cudaStream_t s) {
+  const bool sines = sol == SIPG_SOL_SINSIN || sol == SIPG_SOL_MODES;
+  const int modes_n = sol == SIPG_SOL_MODES ? modes->nmodes : 1;
+  const int nm = !sines ? 0 : (modes_n <= 1 ? 1 : (modes_n <= 4 ? 4 : 8)), n = op->p + 1;
+  const size_t table = (size_t)nm * n * op->dim;
   double* d_axes = nullptr;
-  SIPG_CUDA_TRY(cudaMallocAsync((void**)&d_axes, sizeof(double) * 2 * op->dim, s));
-  k_mesh_axes<<<1, 2, 0, s>>>(d_axes, d_axes + op->dim, op->dim);
-  count_launch();
+  SIPG_CUDA_TRY(cudaMallocAsync((void**)&d_axes, sizeof(double) * (2 * op->dim + 2 * table), s));
+  double *xcol = d_axes, *yrow = d_axes + op->dim, *sx = yrow + op->dim, *sy = sx + table;
+  // the axes' running sums: a chain of dim dependent additions, so on the host
+  // where a copy of them is staged at once (512: 1 us and the copy, against 16
+  // us on the device)
+  cudaError_t err = cudaSuccess;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    cap = cudaStreamCaptureStatusActive;
+  }
+  if (op->dim <= 4096 && cap == cudaStreamCaptureStatusNone) {  // (a captured copy would read the host array later)
+    std::vector<double> xc, yr;
+    mesh_axes(op->dim, xc, yr);
+    xc.insert(xc.end(), yr.begin(), yr.end());
+    err = cudaMemcpyAsync(d_axes, xc.data(), sizeof(double) * xc.size(), cudaMemcpyHostToDevice, s);
+  } else {
+    k_mesh_axes<<<1, 2, 0, s>>>(xcol, yrow, op->dim);
+    count_launch();
+  }
   ProblemArgs pa;
   pa.sol = sol;
   std::memset(&pa.modes, 0, sizeof(pa.modes));
   if (modes) pa.modes = *modes;
   const RhsTables tb = make_rhs_tables(op->tab, op->dim);
   const int threads = 128, blocks = (int)((op->noe + threads - 1) / threads);
-  k_rhs<<<blocks, threads, 0, s>>>(d_b, op->p, op->dim, op->pen, pa, tb, d_axes, d_axes + op->dim);
-  count_launch();
-  SIPG_CUDA_TRY(cudaGetLastError());
-  SIPG_CUDA_TRY(cudaFreeAsync(d_axes, s));
+  if (sines) {
+    const SineModes m = sine_modes(pa);
+    k_sine_tables<<<dim3((op->dim + 63) / 64, nm * n), 64, 0, s>>>(sx, sy, n, op->dim, m, tb, xcol, yrow);
+    if (nm == 1) k_rhs_sines<1><<<blocks, threads, 0, s>>>(d_b, op->p, op->dim, op->pen, m, tb, sx, sy);
+    else if (nm == 4) k_rhs_sines<4><<<blocks, threads, 0, s>>>(d_b, op->p, op->dim, op->pen, m, tb, sx, sy);
+    else k_rhs_sines<8><<<blocks, threads, 0, s>>>(d_b, op->p, op->dim, op->pen, m, tb, sx, sy);
+    count_launch(2);
+  } else {
+    k_rhs<<<blocks, threads, 0, s>>>(d_b, op->p, op->dim, op->pen, pa, tb, xcol, yrow);
+    count_launch();
+  }
+  if (err == cudaSuccess) err = cudaGetLastError();
+  cudaFreeAsync(d_axes, s);
+  SIPG_CUDA_TRY(err);
   return SIPG_OK;
 }
 
