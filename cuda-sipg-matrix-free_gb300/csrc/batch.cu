@@ -111,6 +111,7 @@ struct sipg_batch {
   CgState<float>* h_st32 = nullptr;    // pinned mirrors, n each
   CgState<double>* h_st64 = nullptr;
   cudaStream_t cap = nullptr;
+  LaunchFork fork;  // side streams for the capture's parallel branches
   cudaGraphExec_t exec = nullptr;
   int K = 8;
   unsigned long long graph_launches = 0;  // kernel launches one replay makes
@@ -154,6 +155,7 @@ static void batch_free(sipg_batch* b) {
   cudaFreeHost(b->h_st32);
   cudaFreeHost(b->h_st64);
   if (b->cap) cudaStreamDestroy(b->cap);
+  b->fork.destroy();
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   for (sipg_op* op : b->owned) sipg_op_destroy(op);
@@ -307,17 +309,19 @@ static sipg_status batch_capture(sipg_batch* b) {
   // the launches counted while capturing are the graph's, not executed ones
   const unsigned long long c0 = g_launches.load();
   for (int k = 0; k < b->K && err == cudaSuccess; ++k) {
-    // z = M r (two-level), p = z + beta p, Ap and alpha, then the update
-    if (twolevel_enqueue_batched(b->d_tl, b->tlplan, b->cap) != SIPG_OK) err = cudaErrorUnknown;
+    // z = M r (two-level), p = z + beta p, Ap and alpha, then the update; the
+    // degrees' launches are parallel branches of the graph
+    if (twolevel_enqueue_batched(b->d_tl, b->tlplan, b->cap, &b->fork) != SIPG_OK) err = cudaErrorUnknown;
     if (err != cudaSuccess) break;
     k_fcg_inner_pdirection_batched<<<vg, kVecThreads, 0, b->cap>>>(b->d_vec);
     count_launch();
     err = cudaGetLastError();
-    for (BGroup& g : b->groups) {
-      if (err != cudaSuccess) break;
-      err = launch_apply_batched_f32(g.p, g.cfg32, APPLY_DOT, g.d_cg, g.d_tiles32, (int)g.members.size(), g.total32,
-                                     b->inst[g.members[0]].op->tab, b->cap);
-    }
+    if (err == cudaSuccess)
+      err = b->fork.run(b->cap, (int)b->groups.size(), [&](int k2, cudaStream_t s2) {
+        BGroup& g = b->groups[k2];
+        return launch_apply_batched_f32(g.p, g.cfg32, APPLY_DOT, g.d_cg, g.d_tiles32, (int)g.members.size(), g.total32,
+                                        b->inst[g.members[0]].op->tab, s2);
+      });
     if (err != cudaSuccess) break;
     k_fcg_inner_pupdate_batched<<<vg, kVecThreads, 0, b->cap>>>(b->d_vec);
     count_launch();

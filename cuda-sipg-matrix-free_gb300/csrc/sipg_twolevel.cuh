@@ -39,6 +39,53 @@ struct TlInst {
   TlLev<float> lev[kTlMaxLevels];
 };
 
+// Independent launches side by side within one stream's order: launch k runs on
+// a side stream between two events, so that in a captured graph the launches
+// are parallel branches.  For a batch's per-degree launches, each of which fills
+// a part of the chip: 32 uneven problems of degrees 2..8 (seven launches)
+// measured 55.6 -> 47.0 ms per batched solve.
+struct LaunchFork {
+  std::vector<cudaStream_t> side;
+  std::vector<cudaEvent_t> done;
+  cudaEvent_t start = nullptr;
+  // f(k, stream) for k in [0, n), ordered after s's work so far and before its next
+  template <typename F>
+  cudaError_t run(cudaStream_t s, int n, F f) {
+    if (n <= 1) return n == 1 ? f(0, s) : cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    if (!start) e = cudaEventCreateWithFlags(&start, cudaEventDisableTiming);
+    while (e == cudaSuccess && (int)side.size() < n - 1) {
+      cudaStream_t st = nullptr;
+      e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+      if (e != cudaSuccess) break;
+      side.push_back(st);
+    }
+    while (e == cudaSuccess && (int)done.size() < n - 1) {
+      cudaEvent_t ev = nullptr;
+      e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+      if (e != cudaSuccess) break;
+      done.push_back(ev);
+    }
+    if (e == cudaSuccess) e = cudaEventRecord(start, s);
+    for (int k = 1; k < n && e == cudaSuccess; ++k) {
+      e = cudaStreamWaitEvent(side[k - 1], start, 0);
+      if (e == cudaSuccess) e = f(k, side[k - 1]);
+      if (e == cudaSuccess) e = cudaEventRecord(done[k - 1], side[k - 1]);
+    }
+    if (e == cudaSuccess) e = f(0, s);
+    for (int k = 1; k < n && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(s, done[k - 1], 0);
+    return e;
+  }
+  void destroy() {
+    for (cudaStream_t st : side) cudaStreamDestroy(st);
+    for (cudaEvent_t ev : done) cudaEventDestroy(ev);
+    if (start) cudaEventDestroy(start);
+    side.clear();
+    done.clear();
+    start = nullptr;
+  }
+};
+
 // How a batched application runs: instances in the device array are grouped
 // by degree (group g: [first, first + count)).
 struct TlPlan {
@@ -66,6 +113,7 @@ TlInst twolevel_inst(const void* handle, float* scratch, const float* r, float* 
 TlPlan twolevel_plan(const TlInst* h_insts, const HostTables* const* tabs, int n);
 // Enqueues z = M r for every instance of d_insts (the device copy of the
 // planned array); each instance is skipped once its state says done.
-sipg_status twolevel_enqueue_batched(const TlInst* d_insts, const TlPlan& plan, cudaStream_t s);
+sipg_status twolevel_enqueue_batched(const TlInst* d_insts, const TlPlan& plan, cudaStream_t s,
+                                     LaunchFork* fork = nullptr);
 
 }  // namespace sipg

@@ -1656,26 +1656,33 @@ void tlb_elem_launch(int which, const TlInst* d, const TlPlan::Group& g, cudaStr
 
 // One batched element kernel (0: restriction, 1: finish) for every degree
 // group of the plan.
-void tlb_elem_all(int which, const TlInst* d, const TlPlan& plan, cudaStream_t s) {
-  for (const TlPlan::Group& g : plan.groups) {
+cudaError_t tlb_elem_all(int which, const TlInst* d, const TlPlan& plan, cudaStream_t s, LaunchFork* fork) {
+  auto one = [&](int k, cudaStream_t st) -> cudaError_t {
+    const TlPlan::Group& g = plan.groups[k];
     switch (g.p) {
-      case 1: tlb_elem_launch<1>(which, d, g, s); break;
-      case 2: tlb_elem_launch<2>(which, d, g, s); break;
-      case 3: tlb_elem_launch<3>(which, d, g, s); break;
-      case 4: tlb_elem_launch<4>(which, d, g, s); break;
-      case 5: tlb_elem_launch<5>(which, d, g, s); break;
-      case 6: tlb_elem_launch<6>(which, d, g, s); break;
-      case 7: tlb_elem_launch<7>(which, d, g, s); break;
-      case 8: tlb_elem_launch<8>(which, d, g, s); break;
+      case 1: tlb_elem_launch<1>(which, d, g, st); break;
+      case 2: tlb_elem_launch<2>(which, d, g, st); break;
+      case 3: tlb_elem_launch<3>(which, d, g, st); break;
+      case 4: tlb_elem_launch<4>(which, d, g, st); break;
+      case 5: tlb_elem_launch<5>(which, d, g, st); break;
+      case 6: tlb_elem_launch<6>(which, d, g, st); break;
+      case 7: tlb_elem_launch<7>(which, d, g, st); break;
+      case 8: tlb_elem_launch<8>(which, d, g, st); break;
     }
-  }
-  count_launch(plan.groups.size());
+    return cudaGetLastError();
+  };
+  const int n = (int)plan.groups.size();
+  count_launch(n);
+  if (fork) return fork->run(s, n, one);
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < n && e == cudaSuccess; ++k) e = one(k, s);
+  return e;
 }
 
-sipg_status twolevel_enqueue_batched(const TlInst* d, const TlPlan& plan, cudaStream_t s) {
+sipg_status twolevel_enqueue_batched(const TlInst* d, const TlPlan& plan, cudaStream_t s, LaunchFork* fork) {
   if (plan.n == 0) return SIPG_OK;
   const int n = plan.n;
-  tlb_elem_all(0, d, plan, s);
+  SIPG_CUDA_TRY(tlb_elem_all(0, d, plan, s, fork));
   auto tiles = [&](int l, int tile) {
     const int t = tl_tiles(plan.side_max[l], tile);
     return dim3(t * t, n);
@@ -1690,7 +1697,7 @@ sipg_status twolevel_enqueue_batched(const TlInst* d, const TlPlan& plan, cudaSt
     k_tlb_up<<<tiles(l, kTlUp), kTlTileThreads, 0, s>>>(d, l);
     count_launch();
   }
-  tlb_elem_all(1, d, plan, s);
+  SIPG_CUDA_TRY(tlb_elem_all(1, d, plan, s, fork));
   SIPG_CUDA_TRY(cudaGetLastError());
   return SIPG_OK;
 }
