@@ -52,7 +52,10 @@ __device__ __forceinline__ A block_sum(A v, A* sh) {
   A s = A(0);
   if (t < 32) {
     s = (t < NT / 32) ? sh[t] : A(0);
-    s = warp_sum(s);
+    constexpr int kW = NT / 32;  // the warps' sums: only the steps that meet them
+    constexpr int kTop = kW > 16 ? 16 : (kW > 8 ? 8 : (kW > 4 ? 4 : (kW > 2 ? 2 : (kW > 1 ? 1 : 0))));
+#pragma unroll
+    for (int o = kTop; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   }
   return s;
 }

@@ -114,16 +114,27 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
     return gx >= 0 && gx < dim && gy >= 0 && gy < dim;
   };
   // ---- phase 0: values and magnitudes ----------------------------------------
-  for (int idx = t; idx < NSLOT * NN; idx += NT) {
-    const int k = idx / NSLOT, sl = idx - k * NSLOT;
+  // (every load of the thread first, so that they are in flight together)
+  constexpr int IT = (NSLOT * NN + NT - 1) / NT;
+  double vr[IT], vp[IT];
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int idx = t + it * NT, k = idx / NSLOT, sl = idx - k * NSLOT;
     const int sy = sl / SX, sx = sl - sy * SX;
-    double v = 0.0;
-    if (!corner(sx, sy) && in_mesh(sx, sy)) {
+    vr[it] = vp[it] = 0.0;
+    if (idx < NSLOT * NN && !corner(sx, sy) && in_mesh(sx, sy)) {
       const size_t gk = (size_t)k * noe + (size_t)(y0 - 1 + sy) * dim + (x0 - 1 + sx);
-      v = ldin(a.in + gk);
-      if (MODE == APPLY_CG && !first) v = fma(beta, ldin(pold + gk), v);
-      atomicMax(&sm.mag[sl], fx_mag(v));
+      vr[it] = ldin(a.in + gk);
+      if (MODE == APPLY_CG && !first) vp[it] = ldin(pold + gk);
     }
+  }
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int idx = t + it * NT, k = idx / NSLOT, sl = idx - k * NSLOT;
+    const int sy = sl / SX, sx = sl - sy * SX;
+    if (idx >= NSLOT * NN) break;
+    const double v = MODE == APPLY_CG && !first ? fma(beta, vp[it], vr[it]) : vr[it];
+    if (fx_mag(v) != 0) atomicMax(&sm.mag[sl], fx_mag(v));
     sm.us[sl * NN + k] = make_int2(__double2loint(v), __double2hiint(v));
     if (sx > 0 && sx < SX - 1 && sy > 0 && sy < SY - 1) sm.own[k * NE + (sy - 1) * EX + sx - 1] = v;
   }
