@@ -162,15 +162,22 @@ def _check(status, what=""):
 
 
 def _ptr(t):
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
+
+
+_raw_stream = None  # device index -> handle of its current stream, without building a Stream object
 
 
 def _stream(stream=None):
     if stream is not None:
-        return C.c_void_p(stream)
+        return stream
+    global _raw_stream
     import torch
 
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    if _raw_stream is None:
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+            lambda device: torch.cuda.current_stream(device).cuda_stream)
+    return _raw_stream(torch.cuda.current_device())
 
 
 def selftest_barrier_timeout():
@@ -321,8 +328,6 @@ class Operator:
             pass
 
     def _vec(self, t, dtype=None):
-        import torch
-
         assert t.is_cuda and t.is_contiguous() and t.numel() == self.ndof, "expected a contiguous CUDA vector"
         if dtype is not None:
             assert t.dtype == dtype
@@ -341,8 +346,11 @@ class Operator:
         if out is None:
             out = torch.empty_like(x)
         self._vec(out, x.dtype)
-        f = lib().sipg_apply_f64 if x.dtype == torch.float64 else lib().sipg_apply_f32
-        _check(f(self._h, _ptr(x), _ptr(out), _stream(stream)), "apply")
+        L = _lib or lib()
+        st = (L.sipg_apply_f64 if x.dtype == torch.float64 else L.sipg_apply_f32)(self._h, x.data_ptr(), out.data_ptr(),
+                                                                                 _stream(stream))
+        if st:
+            _check(st, "apply")
         return out
 
     def apply_pairs(self, x, out=None, stream=None):
