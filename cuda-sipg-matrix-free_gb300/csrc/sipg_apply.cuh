@@ -596,6 +596,15 @@ const ApplyTab<T, P>& apply_tabs(const HostTables& h) {
   return t;
 }
 
+// Threads per element of the fixed-point tile: two from p = 6 on, where shared
+// memory leaves 6 to 8 warps per SM at one; they share the element's columns,
+// faces and conversions.
+__host__ __device__ constexpr int fx_split(int p) { return p >= 6 ? 2 : 1; }
+template <typename T, int P>
+constexpr int apply_split() {
+  return sizeof(T) == 8 ? fx_split(P) : 1;
+}
+
 // Shared memory of the fixed-point tile: the elements' parity-form values
 // [NN][TE]; w times their four faces' normal derivatives [4][N1][RS] (LEFT,
 // RIGHT, DOWN, UP), each with the one of the TX or TY elements around the tile
@@ -619,7 +628,7 @@ template <typename T, int P, int TX, int TY>
 constexpr int apply_min_blocks() {
   if constexpr (sizeof(T) == 8) {
     const int smem = (int)((227 * 1024) / (FxSmem<P, TX, TY>::bytes + 2048));
-    const int regs = 65536 / (TX * TY * (P == 1 ? 64 : (P == 2 ? 80 : 128)));
+    const int regs = 65536 / (TX * TY * fx_split(P) * (P == 1 ? 64 : (P == 2 ? 80 : 128)));
     const int m = smem < regs ? smem : regs;
     return m < 1 ? 1 : m;
   }
@@ -639,7 +648,7 @@ __device__ __forceinline__ void apply_block(const ApplyArgs<T>& a, const ApplyTa
 }
 
 template <typename T, int P, int TX, int TY, int MODE>
-__global__ void __launch_bounds__(TX* TY, apply_min_blocks<T, P, TX, TY>())
+__global__ void __launch_bounds__(TX* TY* apply_split<T, P>(), apply_min_blocks<T, P, TX, TY>())
     k_sipg_apply(const __grid_constant__ ApplyArgs<T> a, const __grid_constant__ ApplyTab<T, P> tb) {
   apply_block<T, P, TX, TY, MODE>(a, tb, blockIdx.x, blockIdx.y, blockIdx.y * gridDim.x + blockIdx.x,
                                  gridDim.x * gridDim.y);
@@ -650,7 +659,7 @@ __global__ void __launch_bounds__(TX* TY, apply_min_blocks<T, P, TX, TY>())
 // (the instances' tiles concatenated; each instance reduces into its own
 // scratch and state, and a converged instance's blocks return at once).
 template <typename T, int P, int TX, int TY, int MODE>
-__global__ void __launch_bounds__(TX* TY, apply_min_blocks<T, P, TX, TY>())
+__global__ void __launch_bounds__(TX* TY* apply_split<T, P>(), apply_min_blocks<T, P, TX, TY>())
     k_sipg_apply_batched(const ApplyArgs<T>* __restrict__ insts, const int* __restrict__ tile_start, int ninst,
                          const __grid_constant__ ApplyTab<T, P> tb) {
   const int g = blockIdx.x;
@@ -669,7 +678,7 @@ __global__ void __launch_bounds__(TX* TY, apply_min_blocks<T, P, TX, TY>())
 template <typename T, int P, int TX, int TY>
 cudaError_t launch_apply_tile(int mode, const ApplyArgs<T>& a, const ApplyTab<T, P>& tb, cudaStream_t s) {
   const int rows = a.nrows > 0 ? a.nrows : a.dim;
-  const dim3 grid((a.dim + TX - 1) / TX, (rows + TY - 1) / TY), block(TX, TY);
+  const dim3 grid((a.dim + TX - 1) / TX, (rows + TY - 1) / TY), block(TX, TY, apply_split<T, P>());
   const size_t smem = apply_smem<T, P, TX, TY>();
   cudaError_t err = cudaSuccess;
   bool known = mode == APPLY_PREPARE;
@@ -729,7 +738,7 @@ cudaError_t launch_apply_batched_tile(int mode, const ApplyArgs<T>* insts, const
     known = true;
     err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess || mode == APPLY_PREPARE || total_tiles == 0) return;
-    kernel<<<dim3(total_tiles), dim3(TX, TY), smem, s>>>(insts, tile_start, ninst, tb);
+    kernel<<<dim3(total_tiles), dim3(TX, TY, apply_split<T, P>()), smem, s>>>(insts, tile_start, ninst, tb);
     count_launch();
     err = cudaGetLastError();
   };

@@ -115,12 +115,14 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
   constexpr bool kPivot = MODE != BASE;
   constexpr bool kDot = (BASE == APPLY_CG || BASE == APPLY_DOT);
   constexpr bool kRegs = FxForm<P>::regs;
-  constexpr int kHalo = FxSmem<P, TX, TY>::HALO, RS = FxSmem<P, TX, TY>::RS, kWarps = TE / 32;
+  constexpr int ZS = fx_split(P), NT = TE * ZS;  // threads per element, per CTA
+  constexpr int kHalo = FxSmem<P, TX, TY>::HALO, RS = FxSmem<P, TX, TY>::RS, kWarps = NT / 32;
   const FxTab<P>& fx = tabs.fx;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red_sh[32];
   __shared__ int2 s_nu[NE];                                   // nu HB(b) w_b
   __shared__ double s_wnu[NE];
+  __shared__ unsigned s_mag[ZS > 1 ? ZS * TE : 1];
   __shared__ int s_be[(TY + 2) * (TX + 2)];                   // the elements' scales, halo ring included
   __shared__ double s_v0[kPivot ? (TY + 2) * (TX + 2) : 1];   // and pivots
   int2* uf = reinterpret_cast<int2*>(smem_raw);  // values (low word, high word), then limb pairs, in place
@@ -130,7 +132,8 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
   if (kDot) {
     if (*(volatile int*)&a.st->done) return;  // converged: the launch is a no-op
   }
-  const int tx = threadIdx.x, ty = threadIdx.y, t = ty * TX + tx;
+  const int tx = threadIdx.x, ty = threadIdx.y, t = ty * TX + tx;  // the element
+  const int z = ZS > 1 ? threadIdx.z : 0, lt = z * TE + t;         // which of its threads; linear id
   const int dim = a.dim;
   const int x0 = bx * TX, y0 = a.row0 + by * TY;
   const int gx = x0 + tx, gy = y0 + ty;
@@ -172,9 +175,9 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
   };
   const bool large = fx_large_nu(a.nu * fx.wmax, fx.sk);
   bool bad = fx_biased(a.nu) > kFxMaxNu;
-  if (t < NE) {
-    s_wnu[t] = fx.w[t] * a.nu;
-    s_nu[t] = large ? make_int2(0, 0) : fx_nu(fx.w[t] * a.nu, fx.sk);
+  if (lt < NE) {
+    s_wnu[lt] = fx.w[lt] * a.nu;
+    s_nu[lt] = large ? make_int2(0, 0) : fx_nu(fx.w[lt] * a.nu, fx.sk);
   }
 
   // ---- phase 0 --------------------------------------------------------------
@@ -190,10 +193,16 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
     if (kRegs) rv_[kRegs ? k : 0] = v;
     else uf[k * TE + t] = make_int2(__double2loint(v), __double2hiint(v));
   };
+  const double pv = kPivot && act ? ld(0, e) : 0.0;
+  if constexpr (ZS == 1) {
 #pragma unroll(FxForm<P>::load_unroll)
-  for (int k = 0; k < NN; ++k) put_raw(k, act ? ld(k, e) : 0.0);
+    for (int k = 0; k < NN; ++k) put_raw(k, act ? ld(k, e) : 0.0);
+  } else {
+#pragma unroll(FxForm<P>::load_unroll / ZS)
+    for (int k = z; k < NN; k += ZS) put_raw(k, act ? ld(k, e) : 0.0);
+  }
   // the halo elements: element h to lane h / kWarps of warp h % kWarps
-  for (int h = (t & 31) * kWarps + (t >> 5); h < kHalo; h += TE) {
+  for (int h = (lt & 31) * kWarps + (lt >> 5); h < kHalo; h += NT) {
     int hx, hy;
     if (!halo_at(h, hx, hy)) continue;
     const size_t he = (size_t)hy * dim + hx;
@@ -208,18 +217,25 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
     Be(hy - y0, hx - x0) = fx_be(hm);
     if (kPivot) V0(hy - y0, hx - x0) = v0;
   }
-  const double pv = kPivot ? raw(0) : 0.0;
 #pragma unroll(kRegs ? NN : N1)
-  for (int k = 0; k < NN; ++k) {
+  for (int k = z; k < NN; k += ZS) {
     if (kPivot) put_raw(k, __dadd_rn(raw(k), -pv));
     mag = max(mag, fx_mag(raw(k)));
   }
-  // out of the fixed-point range: this tile takes the plain code
-  bad = bad || (mag >> 21) >= (unsigned)kFxMaxExp;
+  // out of the fixed-point range: this tile takes the plain code (a value
+  // below kFxMinExp only where the whole element is)
+  bool small = false;
   if ((mag >> 21) < (unsigned)kFxMinExp) {
 #pragma unroll(kRegs ? NN : 1)
-    for (int k = 0; k < NN; ++k) bad = bad || raw(k) != 0.0;
+    for (int k = z; k < NN; k += ZS) small = small || raw(k) != 0.0;
   }
+  if constexpr (ZS > 1) {
+    s_mag[lt] = mag;
+    __syncthreads();  // the other threads' values, and their magnitude
+    mag = max(mag, s_mag[lt ^ TE]);
+    static_assert(ZS == 2, "one other thread");
+  }
+  bad = bad || (mag >> 21) >= (unsigned)kFxMaxExp || (small && (mag >> 21) < (unsigned)kFxMinExp);
   const int bs = fx_be(mag);
   Be(ty, tx) = bs;
   if (kPivot) {
@@ -230,6 +246,7 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
   for (int i = 0; i < NE; ++i)
 #pragma unroll
     for (int j = 0; j < NE; ++j) {  // mirrored nodes: the quad's slots are its own
+      if (ZS > 1 && (i + j) % ZS != z) continue;
       const bool mi = 2 * i == N, mj = 2 * j == N;
       long long q[4];
       q[0] = fx_fix(raw(i * N1 + j), bs);
@@ -245,14 +262,14 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
   double acc = 0.0;
   const bool plain = __syncthreads_or(bad);
   if (plain) {
-    if (act) acc = plain_element<P, MODE>(a, tabs.t, gx, gy, ld, pnew);
+    if (act && z == 0) acc = plain_element<P, MODE>(a, tabs.t, gx, gy, ld, pnew);
   } else {
 
   // ---- phase 1 --------------------------------------------------------------
   // w times the normal derivatives of the element's four faces, component b of
   // the face in slot b (odd components at the mirrored node)
 #pragma unroll(FxForm<P>::face_unroll)
-  for (int b = 0; b < N1; ++b) {
+  for (int b = z; b < N1; b += ZS) {
     const int wb = b < NE ? b : N - b;
     long long r0, rN;
     fx_derivatives<P>(fx, wb, [&](int k, bool odd) { return uf[((odd ? N - k : k) * N1 + b) * TE + t]; }, r0, rN);
@@ -265,7 +282,7 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
   // the faces of the elements around the tile, one pair of mirrored components
   // per thread: above and right of the tile the 0 side, below and left the N
   // side
-  for (int task = t; task < kHalo * NE; task += TE) {
+  for (int task = lt; task < kHalo * NE; task += NT) {
     const int j = task / kHalo, h = task - j * kHalo;
     int hx, hy;
     if (!halo_at(h, hx, hy)) continue;
@@ -332,14 +349,14 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
       const int2 nu = s_nu[wb];
       const double wnu = s_wnu[wb];
       long long J, Q;
-      {
+      if (ZS == 1 || z == 0) {
         const long long t0 = rt ? X0(b, t + 1) : ht_[b * kHalo + 2 * TX + ty];
         fx_face<kPivot>(large, wnu, nu, fx.sk, rint, true, t0, R(0, b, tr), ber, XN(b, t), R(1, b, t), bs, dr, mult(b),
                         J, Q);
         R(1, b, t) = J;
         R(0, b, tr) = Q;
       }
-      {
+      if (ZS == 1 || z == 1) {
         const long long t0 = ut ? Y0(b, t - TX) : ht_[b * kHalo + tx];
         fx_face<kPivot>(large, wnu, nu, fx.sk, uint_, true, t0, R(2, b, tu), beu, YN(b, t), R(3, b, t), bs, du, mult(b),
                         J, Q);
@@ -350,7 +367,7 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
   }
   // the faces without an N side in the tile: below it (or below the mesh's last row) ...
   const int rows_in = min(TY, dim - y0);
-  for (int q = t; q < TX * N1; q += TE) {
+  for (int q = lt; q < TX * N1; q += NT) {
     const int b = q / TX, c = q - b * TX, wb = b < NE ? b : N - b, el = (rows_in - 1) * TX + c;
     if (x0 + c >= dim) continue;
     const bool in = y0 + rows_in < dim;
@@ -363,7 +380,7 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
     R(2, b, el) = Q;
   }
   // ... and left of it
-  for (int q = t; q < TY * N1; q += TE) {
+  for (int q = lt; q < TY * N1; q += NT) {
     const int b = q / TY, r = q - b * TY, wb = b < NE ? b : N - b, el = r * TX;
     if (y0 + r >= dim) continue;
     const bool in = x0 > 0;
@@ -377,7 +394,7 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
   __syncthreads();
 
   // ---- phase 2 --------------------------------------------------------------
-  if (act) {
+  {
     // the four faces: where J and Q are (component b at + b * RS), and the face's scale
     struct Face {
       const long long *pj, *pq;
@@ -403,7 +420,8 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
       be += max(0, fx_raise(be, fx.sk, m));
     }
     if (be > bs)
-      for (int k = 0; k < NN; ++k) uf[k * TE + t] = fx_shift(uf[k * TE + t], min(be - bs, 63));
+      for (int k = z; k < NN; k += ZS) uf[k * TE + t] = fx_shift(uf[k * TE + t], min(be - bs, 63));
+    if (ZS > 1) __syncthreads();
     const int ex = fx_exp(be, fx.sk);
     auto jump = [&](const Face& f, int b) { return fx_scaled(f.pj[b * RS], be - f.be); };
     auto half_q = [&](const Face& f, int b) {
@@ -526,14 +544,16 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
       }
     };
 #pragma unroll(FxForm<P>::col_unroll)
-    for (int i = 0; i < NO; ++i) columns(i, std::false_type{});
-    if constexpr (NE > NO) columns(NE - 1, std::true_type{});
+    for (int i = z; i < NO; i += ZS)
+      if (act) columns(i, std::false_type{});
+    if constexpr (NE > NO)
+      if (act && z == NO % ZS) columns(NE - 1, std::true_type{});
   }
   }  // !plain
   if (BASE != APPLY_PLAIN) {
-    const double bt = block_sum<double, TE>(acc, red_sh);
+    const double bt = block_sum<double, NT>(acc, red_sh);
     double total;
-    if (grid_sum_last<double, TE>(bt, a.red, bid, nblocks, red_sh, &total) && t == 0)
+    if (grid_sum_last<double, NT>(bt, a.red, bid, nblocks, red_sh, &total) && lt == 0)
       apply_finish<double, BASE>(a.st, total, par);
   }
 }
