@@ -109,7 +109,7 @@ struct KwInSmem {
 // faces alone.
 template <typename T, int P>
 struct NodalInRegs {
-  static constexpr bool value = sizeof(T) == 4 && P <= 6;
+  static constexpr bool value = sizeof(T) == 4 && P <= 7;
 };
 
 template <typename T, int P, int TX, int TY>
@@ -126,7 +126,7 @@ struct ApplySmem {
 // beyond (whose n^2 outputs would not fit in registers).
 template <typename T, int P>
 struct ApplyColumnForm {
-  static constexpr bool value = P >= 7;
+  static constexpr bool value = P >= 8;
   // at p = 8 the unrolled columns take 255 registers and spill: rolled, 444^2
   // takes 109 us instead of 309
   static constexpr int load_unroll = (P + 1) * (P + 1), halo_unroll = P + 1, col_unroll = P >= 8 ? 1 : P + 1;
