@@ -78,21 +78,6 @@ struct TlHat {
 
 __device__ __forceinline__ bool tl_done(const int* done) { return done && *(volatile const int*)done; }
 
-template <typename T>
-__device__ __forceinline__ T tl_stencil(const TlLev<T>& L, const T* __restrict__ x, int vx, int vy) {
-  const int n1 = L.m + 1, nv = n1 * n1, v = vy * n1 + vx;
-  T s = T(0);
-#pragma unroll
-  for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-    for (int dx = -1; dx <= 1; ++dx) {
-      const int ux = vx + dx, uy = vy + dy;
-      if (ux < 0 || uy < 0 || ux > L.m || uy > L.m) continue;
-      s = fma(L.S[((dy + 1) * 3 + (dx + 1)) * nv + v], x[uy * n1 + ux], s);
-    }
-  return s;
-}
-
 // ---- the DG <-> Q1 transfers (one thread per element, 64 per block) ----
 
 // corner sums cp[(a * 2 + b) * noe + e] = sum_{i1,i2} l_a(x_i1) l_b(x_i2) r(i1,i2,e)
@@ -413,15 +398,6 @@ __device__ __forceinline__ T tl_prolong_value(const TlProlong& q, T c00, T c01, 
   return T(0.25) * ((c00 + c01) + (c10 + c11));
 }
 
-// The pre-smoothed iterate plus the prolonged coarse result at fine vertex (ux, uy).
-template <typename T>
-__device__ __forceinline__ T tl_corrected(const TlLev<T>& F, const TlLev<T>& C, int ux, int uy) {
-  const int cn1 = C.m + 1;
-  const TlProlong q = tl_prolong_at(ux, uy, F.m);
-  return F.x[uy * (F.m + 1) + ux] + tl_prolong_value(q, C.y[q.jy0 * cn1 + q.jx0], C.y[q.jy0 * cn1 + q.jx1],
-                                                      C.y[q.jy1 * cn1 + q.jx0], C.y[q.jy1 * cn1 + q.jx1]);
-}
-
 // One up step for the 32 x 32 tile (tx, ty) of fine vertices: with
 // xc = x + P C.y, two damped-Jacobi sweeps
 //   y1 = xc + wd (b - A xc),   F.y = y1 + wd (b - A y1).
@@ -496,29 +472,84 @@ __device__ __forceinline__ void tl_up_body(const TlLev<T>& F, const TlLev<T>& C,
 // The coarse end of the V-cycle in one block: from level l0 (at most
 // kTlTailCells cells per side; its b given, or from the corner sums cp when
 // l0 = 0) down to the coarsest level, its dense solve, and back up to l0's
-// result y.  Every phase is one pass over a level's vertices followed by a
-// block barrier; x1 and the residual live in y on the way down, the
-// corrected iterate and the first post-sweep in y and x on the way up.
+// result y.  Fifteen short passes, each ending in a block barrier: the vectors
+// they pass on live in shared memory (windows with a ring of zeros), a thread's
+// stencil rows in registers and the dense inverse in shared memory, all loaded
+// at the start -- a pass through global memory waited about 1 us for L2 (15.7 us
+// per V-cycle at 512^2, here 12.7).
+constexpr int kTlTailLevels = 3;  // levels of at most 32, 16 and 8 cells per side
+constexpr int kTlTailSteps = ((kTlTailCells + 1) * (kTlTailCells + 1) + kTlTailThreads - 1) / kTlTailThreads;
+
+template <typename T>
+struct TlTailSmem {
+  static constexpr int W = kTlTailCells + 3;  // a window's row: the level's vertices and the ring
+  T x[W * W], y[W * W];                       // one level's source vectors at a time
+  static constexpr int V0 = (kTlTailCells + 1) * (kTlTailCells + 1), V1 = (kTlTailCells / 2 + 1) * (kTlTailCells / 2 + 1),
+                       V2 = (kTlTailCells / 4 + 1) * (kTlTailCells / 4 + 1);
+  T b_[V0 + V1 + V2], xs_[V0 + V1];           // right-hand sides; pre-smoothed iterates
+  __device__ T* b(int q) { return b_ + (q == 0 ? 0 : (q == 1 ? V0 : V0 + V1)); }
+  __device__ T* xs(int q) { return xs_ + (q == 0 ? 0 : V0); }
+  T yc[(kTlTailCells / 2 + 1) * (kTlTailCells / 2 + 1)];         // the coarser level's result
+  T ainv[(kTlCoarsestCells + 1) * (kTlCoarsestCells + 1) * (kTlCoarsestCells + 1) * (kTlCoarsestCells + 1)];
+};
+
+static_assert(sizeof(TlTailSmem<float>) <= 48 * 1024, "no shared-memory opt-in");
+
 template <typename T, typename LevAt>
 __device__ __forceinline__ void tl_tail_body(LevAt lev, int l0, int nl, const T* __restrict__ ainv,
-                                             const T* __restrict__ cp, int dim) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  if (l0 == 0 && cp) {
-    const TlLev<T> F = lev(0);
-    const int n1 = F.m + 1;
-    for (int v = tid; v < n1 * n1; v += nt) F.b[v] = tl_corner_sum(cp, dim, v % n1, v / n1);
-    __syncthreads();
+                                             const T* __restrict__ cp, int dim, TlTailSmem<T>& sm) {
+  constexpr int W = TlTailSmem<T>::W, NS = kTlTailSteps;
+  const int tid = threadIdx.x, nt = kTlTailThreads;
+  // everything from global memory first
+  TlRow<T> rows[kTlTailLevels - 1][NS];
+#pragma unroll
+  for (int q = 0; q < kTlTailLevels - 1; ++q) {
+    const bool have = l0 + q + 1 < nl;
+    const TlLev<T> F = lev(have ? l0 + q : l0);
+    const int nv = (F.m + 1) * (F.m + 1);
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+      const int v = tid + k * nt;
+      const bool ok = have && v < nv;
+      tl_load_row(F, ok ? v : 0, nv, ok, false, rows[q][k]);
+    }
   }
-  for (int l = l0; l + 1 < nl; ++l) {
-    const TlLev<T> F = lev(l), C = lev(l + 1);
-    const int m = F.m, n1 = m + 1, nv = n1 * n1;
-    for (int v = tid; v < nv; v += nt) F.y[v] = F.wd[v] * F.b[v];  // x1
+  {
+    const TlLev<T> F = lev(l0);
+    const int n1 = F.m + 1;
+    for (int v = tid; v < n1 * n1; v += nt)
+      sm.b(0)[v] = (l0 == 0 && cp) ? tl_corner_sum(cp, dim, v % n1, v / n1) : F.b[v];
+    const int cnv = (lev(nl - 1).m + 1) * (lev(nl - 1).m + 1);
+    for (int v = tid; v < cnv * cnv; v += nt) sm.ainv[v] = __ldg(ainv + v);
+  }
+  for (int v = tid; v < W * W; v += nt) sm.x[v] = sm.y[v] = T(0);
+  __syncthreads();
+  // down
+#pragma unroll
+  for (int q = 0; q < kTlTailLevels - 1; ++q) {
+    if (l0 + q + 1 >= nl) break;
+    const int m = lev(l0 + q).m, n1 = m + 1, nv = n1 * n1, cn1 = lev(l0 + q + 1).m + 1;
+    int win[NS];  // the vertex's place in a window
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+      const int v = tid + k * nt;
+      win[k] = v < nv ? (v / n1 + 1) * W + v % n1 + 1 : -1;
+      if (win[k] >= 0) sm.y[win[k]] = rows[q][k].wd * sm.b(q)[v];  // x1
+    }
     __syncthreads();
-    for (int v = tid; v < nv; v += nt) F.x[v] = fma(F.wd[v], F.b[v] - tl_stencil(F, F.y, v % n1, v / n1), F.y[v]);
+#pragma unroll
+    for (int k = 0; k < NS; ++k)
+      if (win[k] >= 0) {
+        const int v = tid + k * nt;
+        const T x = fma(rows[q][k].wd, sm.b(q)[v] - tl_row_apply<T, W>(rows[q][k], sm.y + win[k] - W - 1), sm.y[win[k]]);
+        sm.x[win[k]] = x;
+        sm.xs(q)[v] = x;
+      }
     __syncthreads();
-    for (int v = tid; v < nv; v += nt) F.y[v] = F.b[v] - tl_stencil(F, F.x, v % n1, v / n1);  // residual
+#pragma unroll
+    for (int k = 0; k < NS; ++k)
+      if (win[k] >= 0) sm.y[win[k]] = sm.b(q)[tid + k * nt] - tl_row_apply<T, W>(rows[q][k], sm.x + win[k] - W - 1);
     __syncthreads();
-    const int cn1 = C.m + 1;
     for (int v = tid; v < cn1 * cn1; v += nt) {
       const int J = v % cn1, I = v / cn1;
       T acc = T(0);
@@ -527,32 +558,64 @@ __device__ __forceinline__ void tl_tail_body(LevAt lev, int l0, int nl, const T*
         const T wy = tl_w<T>(iy, I, m);
         for (int ix = 2 * J - 1; ix <= 2 * J + 1; ++ix) {
           if (ix < 0 || ix > m) continue;
-          acc = fma(wy * tl_w<T>(ix, J, m), F.y[iy * n1 + ix], acc);
+          acc = fma(wy * tl_w<T>(ix, J, m), sm.y[(iy + 1) * W + ix + 1], acc);
         }
       }
-      C.b[v] = acc;
+      sm.b(q + 1)[v] = acc;
     }
     __syncthreads();
+    for (int v = tid; v < W * W; v += nt) sm.x[v] = sm.y[v] = T(0);  // the next level's rings
+    __syncthreads();
   }
-  {
+  {  // the coarsest level
+    const int qc = nl - 1 - l0;
     const TlLev<T> L = lev(nl - 1);
     const int nv = (L.m + 1) * (L.m + 1);
     for (int v = tid; v < nv; v += nt) {
       T acc = T(0);
-      for (int u = 0; u < nv; ++u) acc = fma(ainv[v * nv + u], L.b[u], acc);
-      L.y[v] = acc;
+      for (int u = 0; u < nv; ++u) acc = fma(sm.ainv[v * nv + u], sm.b(qc)[u], acc);
+      if (qc == 0) L.y[v] = acc;
+      else sm.yc[v] = acc;
     }
     __syncthreads();
   }
-  for (int l = nl - 2; l >= l0; --l) {
-    const TlLev<T> F = lev(l), C = lev(l + 1);
-    const int n1 = F.m + 1, nv = n1 * n1;
-    for (int v = tid; v < nv; v += nt) F.y[v] = tl_corrected(F, C, v % n1, v / n1);  // xc
+  // up
+#pragma unroll
+  for (int q = kTlTailLevels - 2; q >= 0; --q) {
+    if (l0 + q + 1 >= nl) continue;
+    const TlLev<T> F = lev(l0 + q);
+    const int m = F.m, n1 = m + 1, nv = n1 * n1, cn1 = lev(l0 + q + 1).m + 1;
+    int win[NS];
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+      const int v = tid + k * nt;
+      win[k] = v < nv ? (v / n1 + 1) * W + v % n1 + 1 : -1;
+      if (win[k] >= 0) {  // xc
+        const TlProlong p = tl_prolong_at(v % n1, v / n1, m);
+        sm.y[win[k]] = sm.xs(q)[v] + tl_prolong_value(p, sm.yc[p.jy0 * cn1 + p.jx0], sm.yc[p.jy0 * cn1 + p.jx1],
+                                                      sm.yc[p.jy1 * cn1 + p.jx0], sm.yc[p.jy1 * cn1 + p.jx1]);
+      }
+    }
     __syncthreads();
-    for (int v = tid; v < nv; v += nt) F.x[v] = fma(F.wd[v], F.b[v] - tl_stencil(F, F.y, v % n1, v / n1), F.y[v]);
+#pragma unroll
+    for (int k = 0; k < NS; ++k)
+      if (win[k] >= 0)
+        sm.x[win[k]] = fma(rows[q][k].wd, sm.b(q)[tid + k * nt] - tl_row_apply<T, W>(rows[q][k], sm.y + win[k] - W - 1),
+                           sm.y[win[k]]);
     __syncthreads();
-    for (int v = tid; v < nv; v += nt) F.y[v] = fma(F.wd[v], F.b[v] - tl_stencil(F, F.x, v % n1, v / n1), F.x[v]);
-    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NS; ++k)
+      if (win[k] >= 0) {
+        const int v = tid + k * nt;
+        const T y = fma(rows[q][k].wd, sm.b(q)[v] - tl_row_apply<T, W>(rows[q][k], sm.x + win[k] - W - 1), sm.x[win[k]]);
+        if (q == 0) F.y[v] = y;
+        else sm.yc[v] = y;
+      }
+    if (q > 0) {
+      __syncthreads();
+      for (int v = tid; v < W * W; v += nt) sm.x[v] = sm.y[v] = T(0);
+      __syncthreads();
+    }
   }
 }
 
@@ -589,7 +652,8 @@ __global__ void __launch_bounds__(kTlTailThreads)
     k_tl_tail(const __grid_constant__ TlLevels<T> L, int l0, int nl, const T* __restrict__ ainv,
               const T* __restrict__ cp, int dim, const int* done) {
   if (tl_done(done)) return;
-  tl_tail_body<T>([&](int l) { return L.lev[l]; }, l0, nl, ainv, cp, dim);
+  extern __shared__ __align__(16) unsigned char tail_raw[];
+  tl_tail_body<T>([&](int l) { return L.lev[l]; }, l0, nl, ainv, cp, dim, *reinterpret_cast<TlTailSmem<T>*>(tail_raw));
 }
 
 // The Q1 function of the element's corner values at node (i1, i2).
@@ -748,7 +812,9 @@ __global__ void __launch_bounds__(kTlTileThreads) k_tlb_down(const TlInst* __res
 __global__ void __launch_bounds__(kTlTailThreads) k_tlb_tail(const TlInst* __restrict__ insts) {
   const TlInst& v = insts[blockIdx.y];
   if (tlb_skip(v)) return;
-  tl_tail_body<float>([&](int l) { return v.lev[l]; }, v.tail0, v.nl, v.ainv, v.cp, v.dim);
+  extern __shared__ __align__(16) unsigned char tail_raw[];
+  tl_tail_body<float>([&](int l) { return v.lev[l]; }, v.tail0, v.nl, v.ainv, v.cp, v.dim,
+                      *reinterpret_cast<TlTailSmem<float>*>(tail_raw));
 }
 __global__ void __launch_bounds__(kTlTileThreads) k_tlb_up(const TlInst* __restrict__ insts, int l) {
   const TlInst& v = insts[blockIdx.y];
@@ -1538,7 +1604,7 @@ sipg_status twolevel_enqueue(const sipg_op* op, const void* handle, const float*
   }
   TlLevels<float> levels{};
   for (int l = 0; l < nl; ++l) levels.lev[l] = tl.lev[l];
-  k_tl_tail<float><<<1, kTlTailThreads, 0, s>>>(levels, l0, nl, tl.ainv, tl.cp, dim, done);
+  k_tl_tail<float><<<1, kTlTailThreads, sizeof(TlTailSmem<float>), s>>>(levels, l0, nl, tl.ainv, tl.cp, dim, done);
   count_launch();
   for (int l = l0 - 1; l >= 0; --l) {
     const int t = tl_tiles(tl.lev[l].m + 1, kTlUp);
@@ -1691,7 +1757,7 @@ sipg_status twolevel_enqueue_batched(const TlInst* d, const TlPlan& plan, cudaSt
     k_tlb_down<<<tiles(l + 1, kTlDown), kTlTileThreads, 0, s>>>(d, l);
     count_launch();
   }
-  k_tlb_tail<<<dim3(1, n), kTlTailThreads, 0, s>>>(d);
+  k_tlb_tail<<<dim3(1, n), kTlTailThreads, sizeof(TlTailSmem<float>), s>>>(d);
   count_launch();
   for (int l = plan.max_tail0 - 1; l >= 0; --l) {
     k_tlb_up<<<tiles(l, kTlUp), kTlTileThreads, 0, s>>>(d, l);
