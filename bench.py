@@ -54,8 +54,12 @@ MIXED_INNER_TOL = 3e-2       # the flexible solve's inner tolerance (measured fa
 
 
 def fp64_flops_per_dof(p):
-    """FP64 flops per DoF of one fused FP64 apply of degree p (column form)."""
+    """FP64 flops per DoF of one apply of degree p as FP64 chains (column form).
+    The apply takes its sums as 64-bit integers instead, so a rate in these
+    flops is an equivalent, and may exceed the FP64 pipe's."""
     return 2.0 * (2 * (p + 1) + 8 + 12.0 / (p + 1) + 4.0 / (p + 1) ** 2)
+
+
 METRIC = "GDoF/s per SIPG apply (FP64, 1024x1024 elements, p=4)"
 CONFIG = {
     "workload": "fused SIPG-SEM apply y = A u, 1024x1024 quads, p=4, pen=16, 100 applies per step",
@@ -339,9 +343,10 @@ def run_ours(args):
             "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": traffic, "peak_source": "%s (MEASURED_PEAKS.json hbm_gbs)" % peak_src,
             "algorithmic_bytes_per_dof": BYTES_PER_DOF, "launch_ms": dur * 1e3,
-            "fp64_pipe": {"achieved_tflops": fp64_achieved, "peak_tflops": fp64_peak, "frac": fp64_achieved / fp64_peak,
-                          "flops_per_dof": FP64_FLOPS_PER_DOF,
-                          "peak_source": "measured live (sipg_probe_fma_peak, independent DFMA chains)"},
+            "fp64_equivalent": {"achieved_tflops": fp64_achieved, "fp64_fma_peak_tflops": fp64_peak,
+                                "ratio": fp64_achieved / fp64_peak, "flops_per_dof": FP64_FLOPS_PER_DOF,
+                                "what": "the same sums as FP64 chains; the apply takes them as 64-bit integers",
+                                "peak_source": "measured live (sipg_probe_fma_peak, independent DFMA chains)"},
         },
     }
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
@@ -461,8 +466,8 @@ def _roofline_solve(bytes_total, ms, fp64_applies, ndof, p, fp64_peak):
            "peak_source": "%s (MEASURED_PEAKS.json hbm_gbs)" % src, "algorithmic_bytes": bytes_total}
     if fp64_peak:
         fl = fp64_applies * fp64_flops_per_dof(p) * ndof / (ms * 1e-3) / 1e12
-        out["fp64_pipe"] = {"achieved_tflops": fl, "peak_tflops": fp64_peak, "frac": fl / fp64_peak,
-                            "fp64_applies": fp64_applies}
+        out["fp64_equivalent"] = {"achieved_tflops": fl, "fp64_fma_peak_tflops": fp64_peak, "ratio": fl / fp64_peak,
+                                  "fp64_applies": fp64_applies}
     return out
 
 

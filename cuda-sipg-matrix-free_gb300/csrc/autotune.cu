@@ -5,20 +5,21 @@
 // 32 consecutive values) by TY rows, with one or two threads per element; a
 // CTA holds TX * TY elements and their (p+1)^2 nodal blocks in shared memory.
 // For FP64 on small meshes there is also the per-node tile (a few elements
-// per CTA, one thread per output node), which spreads the thin FP64 pipe's
-// work over many more warps and SMs.
+// per CTA, one thread per output node), which spreads a small mesh's work over
+// many more warps and SMs.
 // TY trades halo overhead (TX + TY halo elements per tile) and reduction
 // partials against shared memory per CTA and so resident CTAs per SM; a
 // second thread per element doubles the resident warps at the same shared
-// memory, which pays where the apply waits on latency (the compensated one)
-// rather than on a pipe (FP64).  The best choice depends on the degree, the
+// memory, which pays where the apply waits on latency (the compensated one;
+// the FP64 one splits its elements in two from p = 6 on by itself).  The best choice depends on the degree, the
 // mesh size (how many waves of CTAs fill the 152 SMs) and the arithmetic.  The
 // tuner times each candidate on the operator itself -- a few applies on
 // scratch vectors -- keeps the fastest, and remembers it for (degree, dim,
 // kind) in a process-wide table that new operators consult at creation.  Every tile
-// shape computes each output from the same operations in the same order, so
-// the apply's result does not depend on the choice (CG reductions sum
-// per-block partials, whose grouping does change with TY).
+// shape computes each output from the same operations (the FP64 sums are exact
+// integers, so their order is free), so the apply's result does not depend on
+// the choice (CG reductions sum per-block partials, whose grouping does change
+// with TY).
 #include <cmath>
 #include <map>
 #include <mutex>

@@ -4,10 +4,12 @@
 // On a mesh of a few hundred elements an iteration of the graph-driven CG
 // (capi.cu) is two short kernels whose cost is launch and reduction latency:
 // 15 us at 16 x 16, p = 4, of which the arithmetic is a fraction.  Here one
-// cooperative launch (every CTA resident) runs all iterations: 12.7 us per
-// iteration there, the rest being the two grid barriers' L2 round trips
-// (fence, arrival, polls, partial reads) that the two reductions of an
-// iteration need.  Per iteration:
+// cooperative launch (every CTA resident) runs all iterations: 11.5 us per
+// iteration there (12.7 with FP64 chains in the apply), the rest being the two
+// grid barriers' L2 round trips (fence, arrival, polls, partial reads) that the
+// two reductions of an iteration need.  One 16-CTA cluster with its barrier and
+// distributed shared memory in place of the grid barrier took 14-18 us: the
+// FP64 vector work then runs on 16 SMs.  Per iteration:
 //   A  the per-node apply of the CTA's tiles with the direction p = r + beta
 //      p_old formed on the fly (the same per-tile code as
 //      k_sipg_apply_pernode), its p.Ap partial stored; grid barrier;

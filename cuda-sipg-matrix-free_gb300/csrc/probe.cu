@@ -1,6 +1,6 @@
 // probe.cu -- diagnostic: the FP64 and FP32 FMA throughput of the current
-// device, measured with independent FMA chains (used to state what fraction of
-// the FP64 pipe the FP64 apply reaches; GB300's FP64 rate is about 1/50 of FP32).
+// device, measured with independent FMA chains (the rate an FP64 kernel's sums
+// are compared with; GB300's FP64 rate is about 1/50 of FP32).
 #include "sipg_internal.cuh"
 
 namespace sipg {

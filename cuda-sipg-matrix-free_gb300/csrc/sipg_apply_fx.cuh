@@ -14,9 +14,16 @@
 // Every output depends on the element and its four neighbours alone, through
 // integers, so every tile shape gives the same bits.
 //
-// Bound by instruction issue: about 120 instructions per DoF at p = 4 (half of
-// them 64-bit products and sums), where the FP64 chains were bound by an FP64
-// pipe of 2 operations per SM and cycle.
+// Bound by integer issue and its latency: 183 instructions per DoF at p = 4 (29
+// of them the products; the rest conversions, parity form, limbs, 64-bit
+// additions and shared memory); ncu: multiply-add pipe 54 %, 46 % of the issue
+// slots with the 16 warps per SM that registers and shared memory allow, where FP64 chains are bound by an FP64
+// pipe of 2 operations per SM and cycle (21 per DoF).  Measured, FP64 chains
+// against this: 1024^2, p = 4 1080 -> 266 us (388 -> 1577 GB/s of the 16 bytes
+// per DoF); 443^2, p = 8 977 -> 288 us; ~16 M DoF, p = 1..8: 25, 26, 25, 24, 22,
+// 20, 18, 16 -> 81, 97, 94, 98, 79, 70, 67, 55 GDoF/s.  The largest error
+// against 64-bit-exact sums fell with it (p = 4: 3.3e-16 -> 2.4e-16 of the
+// largest output).
 #pragma once
 
 #include <type_traits>

@@ -2,13 +2,12 @@
 // output node.
 //
 // GB300 issues FP64 at a small fraction of its FP32 rate: a warp instruction of
-// 32 DFMAs occupies a sub-partition's FP64 unit for tens of cycles.  The
-// element-per-thread apply (sipg_apply.cuh) gives every thread the whole
-// (p+1)^2-output chain of one element, so a mesh with few elements -- 256 at
-// 16 x 16 -- runs a few warps, each through ~1000 dependent-issue DFMAs, on a
-// handful of SMs: tens of microseconds per apply, whatever the tile shape.
-// Here a CTA holds EX x EY elements and gives each output node its own thread:
-// the same operations spread over (p+1)^2 times more warps, on more SMs.
+// 32 conversions or sums occupies a sub-partition's FP64 unit for 64 cycles.
+// The element-per-thread apply (sipg_apply_fx.cuh) gives every thread the whole
+// (p+1)^2 outputs of one element, so a mesh with few elements -- 256 at 16 x 16
+// -- runs a few warps, each through thousands of instructions, on a handful of
+// SMs.  Here a CTA holds EX x EY elements and gives each output node its own
+// thread: the same operations spread over (p+1)^2 times more warps, on more SMs.
 //
 // The sums are the fixed-point ones of sipg_apply_fx.cuh (sipg_fx.cuh): the
 // same integers, whose sums do not depend on their order, so the result is

@@ -110,10 +110,12 @@ enum ApplyMode : int {
   APPLY_RESID = 2,  // y = b - A u; r.r -> rr, stop/done set
   APPLY_DOT = 3,    // y = A p for a direction p formed beforehand (k_cg_direction*); p.Ap -> alpha
   // FP64: APPLY_RESID / APPLY_DOT with every zero-sum contraction taken over
-  // differences from one value of its element line (the FP32 apply always
-  // does this): the residual checks and outer steps of the mixed solvers,
+  // differences from its element's first value (the FP32 apply always takes
+  // them, from one value of the element line): the residual checks and outer steps of the mixed solvers,
   // where a smooth iterate's rounding in the plain sums would put a floor
   // near 1e-10 under the true relative residual at 1024^2, p = 4.  The FP64
+  // sums themselves are exact (sipg_fx.cuh); what a difference saves is the
+  // value's rounding to 55 bits below the element's largest one.  The FP64
   // CG and the plain apply keep the plain sums.  (The per-node FP64 tile of
   // small meshes runs the plain modes for these.)
   APPLY_RESID_PIVOT = 4,

@@ -193,7 +193,7 @@ sipg_status sipg_apply_host_f64(sipg_op* op, const double* h_in, double* h_out, 
  * has the per-node tile: (p+1)^2 threads per element, one per output node,
  * over ex x ey elements per CTA -- ey = 4 at p = 1, else 2; ex = 4 (p <= 2) or
  * 2 (p >= 3), or twice that -- its default for meshes up to 128 x 128, where
- * 32-element rows leave most of GB300's thin FP64 pipes idle.  Every shape
+ * 32-element rows leave most of the SMs idle.  Every shape
  * gives bit-identical apply results; CG reductions regroup.  Tile indices for
  * the three apply kinds: */
 enum { SIPG_TUNE_F64 = 0, SIPG_TUNE_F32 = 1, SIPG_TUNE_PAIRS = 2 /* compensated, pair vectors */ };
@@ -271,7 +271,7 @@ sipg_status sipg_solve_mixed(sipg_op* op, double* d_x, const double* d_b, const 
 /* *rel = ||b - A x|| / ||b|| (||b - A x|| if b = 0), with d_r = b - A x when
  * d_r is not NULL: the true residual, evaluated in FP64 with every zero-sum
  * contraction of the operator taken over differences from one value of its
- * element line.  The plain sums of sipg_apply_f64 round each term at the
+ * element.  The plain sums of sipg_apply_f64 round each term at the
  * scale of x itself; on a smooth solution their rounding alone puts a floor
  * near 1e-10 under the relative residual at 1024^2, p = 4, which this
  * evaluation lowers about dim-fold.  The mixed solvers decide convergence
