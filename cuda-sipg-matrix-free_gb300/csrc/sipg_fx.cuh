@@ -85,8 +85,8 @@ inline int2 fx_limbs(long long f) {
 // 2^59 and rows up to 2^61 (a middle value's coefficient at degree 2 is 32
 // times a corner's).  Their components then stay below 2^61 and limbs below
 // 2^30, and a node's output below 2^62.  Error against extended precision,
-// relative 2-norm over smooth, uniform and normal values at degree 2: 3.3e-16,
-// 8.6e-17, 1.1e-16; with the bounds of degree 3: 1.6e-15, 2.7e-16, 4.3e-16; FP64
+// relative 2-norm over smooth, uniform and normal values at degree 2: 2.2e-16,
+// 8.0e-17, 9.6e-17; with the bounds of degree 3: 1.6e-15, 2.7e-16, 4.3e-16; FP64
 // chains: 2.2e-16, 1.7e-16, 1.5e-16.  The time is the same.
 template <int P>
 inline int fx_scale(double cmax, double l1) {
@@ -341,6 +341,7 @@ __device__ __forceinline__ void fx_face(bool large, double wnu, int2 nu, int sk,
     Q = __double_as_longlong(__hiloint2double(hi != 0 ? hi + (fx_exp(b, sk) << 20) : 0, __double2loint(q)));
   } else {
     FxAcc s = fx_zero();
+    s.hh = 1;  // the half rounds to nearest (rounded down: 3.3e-16 for smooth values at degree 2, now 2.2e-16)
     fx_mac(s, nu, fx_limbs_of(J));
     Q = (r + fx_total(s)) >> 1;
   }
