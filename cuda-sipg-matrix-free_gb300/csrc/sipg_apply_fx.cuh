@@ -41,6 +41,27 @@ struct FxForm {
   static constexpr int face_unroll = (P >= 5) ? 1 : (P + 1);
 };
 
+// Address of value k of the element whose value 0 is at p: one wide product.
+__device__ __forceinline__ const double* fx_addr(const double* p, unsigned noe, int k) {
+  return reinterpret_cast<const double*>(reinterpret_cast<const char*>(p) + (unsigned long long)noe * (8u * (unsigned)k));
+}
+
+// Value k of element e as the operator sees it (CG: p = r + beta p_old).
+// (Passed by value: a closure over the tile's variables, handed to a function
+// that is not inlined, puts them in memory: 443^2, p = 8: 377 us, here 270.)
+template <bool CG>
+struct FxLoad {
+  const double *in, *pold;
+  unsigned noe;
+  double beta;
+  bool first;
+  __device__ __forceinline__ double operator()(int k, size_t e) const {
+    const double r = __ldg(fx_addr(in + e, noe, k));
+    if (CG) return first ? r : fma(beta, __ldg(fx_addr(pold + e, noe, k)), r);
+    return r;
+  }
+};
+
 // The plain FP64 code, for tiles whose values are out of the fixed-point range
 // (sipg_fx.cuh): one thread computes all outputs of element (gx, gy) with FP64
 // sums, reading it and its neighbours through ld(k, element).  Rolled and
@@ -110,6 +131,37 @@ __device__ __noinline__ double plain_element(const ApplyArgs<double>& a, const T
   return acc;
 }
 
+// A large penalty's terms into the outputs that this thread (z of ZS) has
+// stored for element (gx, gy); returns its share of the reduction.  (A pass of
+// its own, off the path of the other penalties: as conditions on it, 5 % there.)
+template <int P, int MODE, int ZS, typename Ld>
+__device__ __noinline__ double add_penalty(const ApplyArgs<double>& a, const Tab<double, P>& tb, int gx, int gy, int z,
+                                           Ld ld, const double* pnew) {
+  constexpr int N = P, N1 = P + 1, BASE = apply_base_mode(MODE);
+  const size_t noe = (size_t)a.dim * a.dim, e = (size_t)gy * a.dim + gx;
+  double acc = 0.0;
+#pragma unroll 1
+  for (int i1 = 0; i1 < N1; ++i1) {
+    if (ZS > 1 && min(i1, N - i1) % ZS != z) continue;  // its columns
+#pragma unroll 1
+    for (int j = 0; j < N1; ++j) {
+      const bool face = i1 == 0 || i1 == N || j == 0 || j == N;
+      if (BASE == APPLY_PLAIN && !face) continue;
+      const size_t gk = (size_t)(i1 * N1 + j) * noe + e;
+      double v = a.out[gk];
+      if (face) {
+        const double q = fx_penalty<P>(tb, a.nu, a.dim, gx, gy, i1, j, ld);
+        v = __dadd_rn(v, BASE == APPLY_RESID ? -q : q);
+        a.out[gk] = v;
+      }
+      if (BASE == APPLY_RESID) acc = fma(v, v, acc);
+      else if (BASE == APPLY_CG) acc = fma(pnew[gk], v, acc);
+      else if (BASE == APPLY_DOT) acc = fma(ld(i1 * N1 + j, e), v, acc);
+    }
+  }
+  return acc;
+}
+
 template <int P, int TX, int TY, int MODE>
 __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const ApplyTab<double, P>& tabs, int bx,
                                               int by, int bid, int nblocks) {
@@ -128,7 +180,6 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red_sh[32];
   __shared__ int2 s_nu[NE];                                   // nu HB(b) w_b
-  __shared__ double s_wnu[NE];
   __shared__ unsigned s_mag[ZS > 1 ? ZS * TE : 1];
   __shared__ int s_be[(TY + 2) * (TX + 2)];                   // the elements' scales, halo ring included
   __shared__ double s_v0[kPivot ? (TY + 2) * (TX + 2) : 1];   // and pivots
@@ -158,15 +209,8 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
   }
   const double* __restrict__ pold = par ? a.pbuf1 : a.pbuf0;
   double* __restrict__ pnew = par ? a.pbuf0 : a.pbuf1;
-  // address of value k of the element whose value 0 is at p: one wide product
-  auto addr = [&](const double* p, int k) {
-    return reinterpret_cast<const double*>(reinterpret_cast<const char*>(p) + (unsigned long long)noe * (8u * (unsigned)k));
-  };
-  auto ld = [&](int k, size_t ee) -> double {
-    const double r = __ldg(addr(a.in + ee, k));
-    if (BASE == APPLY_CG) return first ? r : fma(beta, __ldg(addr(pold + ee, k)), r);
-    return r;
-  };
+  auto addr = [&](const double* p, int k) { return fx_addr(p, noe, k); };
+  const FxLoad<BASE == APPLY_CG> ld{a.in, pold, noe, beta, first};
   // the slot of x index (i, odd) and y index (j, odd): even indices at their
   // node, odd ones at the mirrored node
   auto at = [&](int i, bool io, int j, bool jo) -> int { return ((io ? N - i : i) * N1 + (jo ? N - j : j)) * TE + t; };
@@ -181,9 +225,8 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
     return hx >= 0 && hx < dim && hy >= 0 && hy < dim;
   };
   const bool large = fx_large_nu(a.nu * fx.wmax, fx.sk);
-  bool bad = fx_biased(a.nu) > kFxMaxNu;
+  bool bad = false;
   if (lt < NE) {
-    s_wnu[lt] = fx.w[lt] * a.nu;
     s_nu[lt] = large ? make_int2(0, 0) : fx_nu(fx.w[lt] * a.nu, fx.sk);
   }
 
@@ -354,18 +397,17 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
     for (int b = 0; b < N1; ++b) {
       const int wb = b < NE ? b : N - b;
       const int2 nu = s_nu[wb];
-      const double wnu = s_wnu[wb];
       long long J, Q;
       if (ZS == 1 || z == 0) {
         const long long t0 = rt ? X0(b, t + 1) : ht_[b * kHalo + 2 * TX + ty];
-        fx_face<kPivot>(large, wnu, nu, fx.sk, rint, true, t0, R(0, b, tr), ber, XN(b, t), R(1, b, t), bs, dr, mult(b),
+        fx_face<kPivot>(nu, rint, true, t0, R(0, b, tr), ber, XN(b, t), R(1, b, t), bs, dr, mult(b),
                         J, Q);
         R(1, b, t) = J;
         R(0, b, tr) = Q;
       }
       if (ZS == 1 || z == 1) {
         const long long t0 = ut ? Y0(b, t - TX) : ht_[b * kHalo + tx];
-        fx_face<kPivot>(large, wnu, nu, fx.sk, uint_, true, t0, R(2, b, tu), beu, YN(b, t), R(3, b, t), bs, du, mult(b),
+        fx_face<kPivot>(nu, uint_, true, t0, R(2, b, tu), beu, YN(b, t), R(3, b, t), bs, du, mult(b),
                         J, Q);
         R(3, b, t) = J;
         R(2, b, tu) = Q;
@@ -380,7 +422,7 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
     const bool in = y0 + rows_in < dim;
     const int eN = rows_in < TY ? el + TX : TE + c;
     long long J, Q;
-    fx_face<kPivot>(large, s_wnu[wb], s_nu[wb], fx.sk, true, in, Y0(b, el), R(2, b, el), Be(rows_in - 1, c),
+    fx_face<kPivot>(s_nu[wb], true, in, Y0(b, el), R(2, b, el), Be(rows_in - 1, c),
                     ht_[b * kHalo + TX + c], R(3, b, eN), in ? Be(TY, c) : 0, delta(true, rows_in - 1, c, in, TY, c),
                     mult(b), J, Q);
     R(3, b, eN) = J;
@@ -392,7 +434,7 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
     if (y0 + r >= dim) continue;
     const bool in = x0 > 0;
     long long J, Q;
-    fx_face<kPivot>(large, s_wnu[wb], s_nu[wb], fx.sk, true, in, X0(b, el), R(0, b, el), Be(r, 0),
+    fx_face<kPivot>(s_nu[wb], true, in, X0(b, el), R(0, b, el), Be(r, 0),
                     ht_[b * kHalo + 2 * TX + TY + r], R(1, b, TE + r), in ? Be(r, -1) : 0,
                     delta(true, r, 0, in, r, -1), mult(b), J, Q);
     R(1, b, TE + r) = J;
@@ -416,25 +458,13 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
     const Face fd{&R(3, 0, ty < TY - 1 ? t + TX : TE + tx), &R(2, 0, t), scale(gy < dim - 1, ty + 1, tx)};
     const Face fu{&R(3, 0, t), &R(2, 0, ty > 0 ? t - TX : TE + tx), scale(gy > 0, ty - 1, tx)};
     // the outputs' scale; where it is not the element's own, its values move to it
-    int be = max(bs, max(max(fl.be, fr.be), max(fd.be, fu.be)) - (kPivot ? 1 : kFxRoom));
-    if (large) {
-      unsigned m = 0;
-#pragma unroll 1
-      for (int b = 0; b < N1; ++b)
-        m = max(m, max(max(fx_mag(__longlong_as_double(fl.pq[b * RS])), fx_mag(__longlong_as_double(fr.pq[b * RS]))),
-                       max(fx_mag(__longlong_as_double(fd.pq[b * RS])),
-                           fx_mag(__longlong_as_double(fu.pq[b * RS])))));
-      be += max(0, fx_raise(be, fx.sk, m));
-    }
+    const int be = max(bs, max(max(fl.be, fr.be), max(fd.be, fu.be)) - (kPivot ? 1 : kFxRoom));
     if (be > bs)
       for (int k = z; k < NN; k += ZS) uf[k * TE + t] = fx_shift(uf[k * TE + t], min(be - bs, 63));
     if (ZS > 1) __syncthreads();
     const int ex = fx_exp(be, fx.sk);
     auto jump = [&](const Face& f, int b) { return fx_scaled(f.pj[b * RS], be - f.be); };
-    auto half_q = [&](const Face& f, int b) {
-      const long long q = f.pq[b * RS];
-      return large ? fx_units(__longlong_as_double(q), ex) : fx_scaled(q, be - f.be);
-    };
+    auto half_q = [&](const Face& f, int b) { return fx_scaled(f.pq[b * RS], be - f.be); };
     // what the even / odd columns lift from the x faces
     int2 xm[N1], xp[N1];
 #pragma unroll
@@ -556,6 +586,7 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
     if constexpr (NE > NO)
       if (act && z == NO % ZS) columns(NE - 1, std::true_type{});
   }
+    if (large && act) acc = add_penalty<P, MODE, ZS>(a, tabs.t, gx, gy, z, ld, pnew);
   }  // !plain
   if (BASE != APPLY_PLAIN) {
     const double bt = block_sum<double, NT>(acc, red_sh);

@@ -64,7 +64,6 @@ struct PernodeFxSmem {
   int xbe[S::EY * (S::EX + 1)], ybe[S::EX * (S::EY + 1)];  // of the faces
   FxTab<P> fx;
   int2 nu[FxTab<P>::NE];
-  double wnu[FxTab<P>::NE];
   bool large;
 };
 
@@ -80,7 +79,6 @@ __device__ __forceinline__ void pernode_fx_tables(PernodeFxSmem<P, SHAPE>& sm, c
   for (int k = t; k < PernodeFxSmem<P, SHAPE>::NSLOT; k += PernodeShape<P, SHAPE>::NT) sm.mag[k] = 0;
   const bool large = fx_large_nu(nu * fx.wmax, fx.sk);
   if (t < FxTab<P>::NE) {
-    sm.wnu[t] = fx.w[t] * nu;
     sm.nu[t] = large ? make_int2(0, 0) : fx_nu(fx.w[t] * nu, fx.sk);
   }
   if (t == 0) sm.large = large;
@@ -107,6 +105,10 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
   const int dim = a.dim;
   const size_t noe = (size_t)dim * dim;
   auto ldin = [&](const double* p) -> double { return kCoherent ? __ldcg(p) : __ldg(p); };
+  auto ld = [&](int k, size_t e) -> double {
+    const double v = ldin(a.in + (size_t)k * noe + e);
+    return MODE == APPLY_CG && !first ? fma(beta, ldin(pold + (size_t)k * noe + e), v) : v;
+  };
   auto corner = [](int sx, int sy) { return (sx == 0 || sx == SX - 1) && (sy == 0 || sy == SY - 1); };
   auto in_mesh = [&](int sx, int sy) {
     const int gx = x0 - 1 + sx, gy = y0 - 1 + sy;
@@ -139,7 +141,7 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
   }
   __syncthreads();
   // ---- phase 1: parity form ---------------------------------------------------
-  bool bad = fx_biased(a.nu) > kFxMaxNu;
+  bool bad = false;
   for (int sl = t; sl < NSLOT; sl += NT) {
     const unsigned b = sm.mag[sl] >> 21;
     bad = bad || b >= (unsigned)kFxMaxExp;
@@ -170,10 +172,6 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
   }
   if (__syncthreads_or(bad)) {  // out of the fixed-point range: the plain code, one element per thread
     double r = 0.0;
-    auto ld = [&](int k, size_t e) -> double {
-      const double v = ldin(a.in + (size_t)k * noe + e);
-      return MODE == APPLY_CG && !first ? fma(beta, ldin(pold + (size_t)k * noe + e), v) : v;
-    };
     if (t < NE && x0 + t % EX < dim && y0 + t / EX < dim)
       r = plain_element<P, MODE>(a, tabs.t, x0 + t % EX, y0 + t / EX, ld, pnew);
     for (int sl = t; sl < NSLOT; sl += NT) sm.mag[sl] = 0;
@@ -223,7 +221,7 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
     const int ke = x ? b : b * N1, ko = x ? N * N1 + b : b * N1 + N;
     const int be0 = sm.be[s0], beN = sm.be[sN];
     long long J, Q;
-    fx_face<false>(sm.large, sm.wnu[wb], sm.nu[wb], fx.sk, zv, nv, fx_trace0(u0[ke], u0[ko]),
+    fx_face<false>(sm.nu[wb], zv, nv, fx_trace0(u0[ke], u0[ko]),
                    sm.r0[i0], be0, fx_traceN(uN[ke], uN[ko]), sm.rN[iN], beN, 0.0, 0, J, Q);
     const int bf = !zv ? beN : (!nv ? be0 : max(be0, beN));
     if (x) {
@@ -247,15 +245,7 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
       const int bs = sm.be[sl];
       const int fL = ey * (EX + 1) + ex, fR = fL + 1, fU = ey * EX + ex, fD = fU + EX;  // faces
       const int bL = sm.xbe[fL], bR = sm.xbe[fR], bU = sm.ybe[fU], bD = sm.ybe[fD];
-      int be = max(bs, max(max(bL, bR), max(bD, bU)) - kFxRoom);
-      if (sm.large) {
-        unsigned m = 0;
-        for (int b = 0; b < N1; ++b) {
-          m = max(m, max(fx_mag(__longlong_as_double(sm.xq[fL * N1 + b])), fx_mag(__longlong_as_double(sm.xq[fR * N1 + b]))));
-          m = max(m, max(fx_mag(__longlong_as_double(sm.yq[fD * N1 + b])), fx_mag(__longlong_as_double(sm.yq[fU * N1 + b]))));
-        }
-        be += max(0, fx_raise(be, fx.sk, m));
-      }
+      const int be = max(bs, max(max(bL, bR), max(bD, bU)) - kFxRoom);
       const int so = be - bs, xp = fx_exp(be, fx.sk);
       auto own = [&](int kk) { return so > 0 ? fx_shift(u[kk], min(so, 63)) : u[kk]; };
       const bool oa = ka >= HE, ob = kb >= HE;  // odd indices sit at the mirrored slots
@@ -276,9 +266,7 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
       fx_mac(s, (oa ? fx.lo : fx.le)[ia * HE + ib], fx_limbs_of(oa ? jl + jr : jl - jr));
       fx_mac(s, (ob ? fx.lo : fx.le)[ib * HE + ia], fx_limbs_of(ob ? jd + ju : jd - ju));
       long long r = fx_total(s);
-      auto half_q = [&](long long q, int bf) {
-        return sm.large ? fx_units(__longlong_as_double(q), xp) : fx_scaled(q, be - bf);
-      };
+      auto half_q = [&](long long q, int bf) { return fx_scaled(q, be - bf); };
       if (ia == 0) {
         const long long ql = half_q(sm.xq[fL * N1 + kb], bL), qr = half_q(sm.xq[fR * N1 + kb], bR);
         r += oa ? ql + qr : ql - qr;
@@ -308,7 +296,9 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
       };
       long long r = row(i);
       if (2 * i != N) r = i1 == i ? r + row(N - i) : r - row(N - i);
-      const double v = fx_double(r, sm.bo[le]);
+      double v = fx_double(r, sm.bo[le]);
+      if (sm.large && (i1 == 0 || i1 == N || j == 0 || j == N))
+        v = __dadd_rn(v, fx_penalty<P>(tabs.t, a.nu, dim, gx, gy, i1, j, ld));
       const size_t gk = (size_t)k * noe + (size_t)gy * dim + gx;
       if (MODE == APPLY_RESID) {
         const double rv = __ldg(a.b + gk) - v;
