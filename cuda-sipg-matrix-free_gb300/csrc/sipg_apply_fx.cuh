@@ -11,8 +11,10 @@
 //      stiffness sums as one fixed-point sum per parity component, the face
 //      terms of index 0 added, back to the nodes, and rounded to a double; then
 //      the epilogue (store; in the CG modes a deterministic grid reduction).
+//   3  the elements that one scale does not fit (sipg_fx.cuh), by FP64 chains.
 // Every output depends on the element and its four neighbours alone, through
-// integers, so every tile shape gives the same bits.
+// integers or through the chain of chain_node, so every tile shape gives the
+// same bits.
 //
 // Bound by integer issue and its latency: 183 instructions per DoF at p = 4 (29
 // of them the products; the rest conversions, parity form, limbs, 64-bit
@@ -36,7 +38,7 @@ namespace sipg {
 template <int P>
 struct FxForm {
   static constexpr bool regs = P <= 4;  // raw values in registers between load and conversion
-  static constexpr int load_unroll = (P >= 5) ? 2 * (P + 1) : (P + 1) * (P + 1);
+  static constexpr int row_unroll = fx_split(P) > 1 ? 1 : 2;  // rows of loads in flight, beyond that
   static constexpr int col_unroll = (P >= 5) ? 1 : (P + 1);
   static constexpr int face_unroll = (P >= 5) ? 1 : (P + 1);
 };
@@ -49,114 +51,235 @@ __device__ __forceinline__ const double* fx_addr(const double* p, unsigned noe, 
 // Value k of element e as the operator sees it (CG: p = r + beta p_old).
 // (Passed by value: a closure over the tile's variables, handed to a function
 // that is not inlined, puts them in memory: 443^2, p = 8: 377 us, here 270.)
-template <bool CG>
+template <bool CG, bool COHERENT>
 struct FxLoad {
   const double *in, *pold;
   unsigned noe;
   double beta;
   bool first;
+  __device__ __forceinline__ double at(const double* p) const { return COHERENT ? __ldcg(p) : __ldg(p); }
   __device__ __forceinline__ double operator()(int k, size_t e) const {
-    const double r = __ldg(fx_addr(in + e, noe, k));
-    if (CG) return first ? r : fma(beta, __ldg(fx_addr(pold + e, noe, k)), r);
+    const double r = at(fx_addr(in + e, noe, k));
+    if (CG) return first ? r : fma(beta, at(fx_addr(pold + e, noe, k)), r);
     return r;
   }
 };
 
-// The plain FP64 code, for tiles whose values are out of the fixed-point range
-// (sipg_fx.cuh): one thread computes all outputs of element (gx, gy) with FP64
-// sums, reading it and its neighbours through ld(k, element).  Rolled and
-// unshared: it is as slow as it is rare.  Returns the thread's share of the
-// reduction.
-template <int P, int MODE, typename Ld>
-__device__ __noinline__ double plain_element(const ApplyArgs<double>& a, const Tab<double, P>& tb, int gx, int gy,
-                                             Ld ld, double* pnew) {
-  constexpr int N = P, N1 = P + 1, BASE = apply_base_mode(MODE);
-  constexpr bool kDot = (BASE == APPLY_CG || BASE == APPLY_DOT);
-  const int dim = a.dim;
-  const size_t noe = (size_t)dim * dim, e = (size_t)gy * dim + gx;
-  // J and Q of the LEFT, RIGHT, DOWN and UP face
+// v + sum_i c(i) l(i) as one FP64 chain; PIVOT: over the differences l(i) - l(0).
+// U: terms whose loads are in flight together.
+template <int P, bool PIVOT, int U, typename C, typename V>
+__device__ __forceinline__ double chain_sum(double v, C c, V l) {
+  const double p0 = PIVOT ? l(0) : 0.0;
+#pragma unroll(U)
+  for (int i = 0; i <= P; ++i) v = fma(c(i), PIVOT ? l(i) - p0 : l(i), v);
+  return v;
+}
+
+// One side of a face for the FP64 chains: its trace and normal derivative (D) at
+// node q of the face of element e (x: an x face; last: the N side).
+template <int P, bool PIVOT, int U, typename Ld>
+__device__ __forceinline__ void chain_side(const double* D, bool x, bool last, int q, size_t e, Ld ld, double& u,
+                                           double& d) {
+  auto line = [&](int i) { return ld(x ? i * (P + 1) + q : q * (P + 1) + i, e); };
+  u = line(last ? P : 0);
+  d = chain_sum<P, PIVOT, U>(0.0, [&](int i) { return D[i]; }, line);
+}
+
+// The neighbour across face f (LEFT, RIGHT, DOWN, UP) of element (gx, gy) = e.
+__device__ __forceinline__ bool chain_across(int f, int dim, int gx, int gy, size_t e, size_t& ne) {
+  ne = f == 0 ? e - 1 : (f == 1 ? e + 1 : (f == 2 ? e + dim : e - dim));
+  return f == 0 ? gx > 0 : (f == 1 ? gx < dim - 1 : (f == 2 ? gy < dim - 1 : gy > 0));
+}
+
+// Output (i1, j) of element (gx, gy) as one FP64 chain: the face terms, the x
+// faces' lift, the row's and the column's stiffness sums, the y faces' lift.
+// PIVOT: zero-sum rows over differences from the line's first value.
+template <int P, bool PIVOT, int U, typename Ld>
+__device__ __forceinline__ double chain_node(const Tab<double, P>* tb, double nu, int dim, int gx, int gy, int i1,
+                                             int j, Ld ld) {
+  constexpr int N = P, N1 = P + 1;
+  const size_t e = (size_t)gy * dim + gx;
+  double J[4], Q[4];  // at the node's line
+#pragma unroll
+  for (int f = 0; f < 4; ++f) {
+    const bool x = f < 2, zero = (f & 1) == 0;  // zero: this element is the 0 side
+    const int q = x ? j : i1, k0 = x ? q : q * N1, kN = x ? N * N1 + q : q * N1 + N;
+    size_t ne;
+    const bool in = chain_across(f, dim, gx, gy, e, ne);
+    const double own = ld(zero ? k0 : kN, e), other = in ? ld(zero ? kN : k0, ne) : 0.0;
+    J[f] = mul_rn(in ? tb->WH[q] : tb->w[q], zero ? own - other : other - own);
+    Q[f] = 0.0;
+  }
+#pragma unroll
+  for (int d = 0; d < 2; ++d) {  // the x face, the y face that the node lies on
+    const bool x = d == 0;
+    const int at = x ? i1 : j, q = x ? j : i1, f = 2 * d + (at == 0 ? 0 : 1);
+    if (at != 0 && at != N) continue;
+    const bool zero = at == 0;
+    size_t ne;
+    const bool in = chain_across(f, dim, gx, gy, e, ne);
+    double u0 = 0.0, d0 = 0.0, uN = 0.0, dN = 0.0, unused, v;
+    chain_side<P, PIVOT, U>(zero ? tb->D0 : tb->DN, x, !zero, q, e, ld, zero ? u0 : uN, zero ? d0 : dN);
+    if (in) chain_side<P, PIVOT, U>(zero ? tb->DN : tb->D0, x, zero, q, ne, ld, zero ? uN : u0, zero ? dN : d0);
+    face_combine<double>(tb->w[q], tb->WH[q], nu, in, u0, d0, uN, dN, unused, v);
+    Q[2 * d + 0] = zero ? v : 0.0;
+    Q[2 * d + 1] = zero ? 0.0 : v;
+  }
+  double v = face_seed<double, N>(i1, j, Q[0], Q[1], Q[2], Q[3]);
+  v = fma(tb->D0[i1], J[0], fma(tb->DN[i1], J[1], v));
+  v = chain_sum<P, PIVOT, U>(v, [&](int i) { return tb->KW[(i1 * N1 + i) * N1 + j]; },
+                             [&](int i) { return ld(i * N1 + j, e); });
+  v = chain_sum<P, PIVOT, U>(v, [&](int i) { return tb->KW[(j * N1 + i) * N1 + i1]; },
+                             [&](int i) { return ld(i1 * N1 + i, e); });
+  v = fma(tb->D0[j], J[2], v);
+  return fma(tb->DN[j], J[3], v);
+}
+
+// A generic pointer to the tables in the kernel's parameters: lanes that index
+// them differently read them like global memory, where the constant bank would
+// serve one address at a time.
+template <int P>
+__device__ __forceinline__ const Tab<double, P>* generic_tab(const Tab<double, P>& tb) {
+  const Tab<double, P>* p = &tb;
+  asm volatile("" : "+l"(p));
+  return p;
+}
+
+// Stores output k of element e, whose value is v, as the mode does, and adds
+// its share of the reduction.
+template <int MODE, typename Ld>
+__device__ __forceinline__ void chain_emit(const ApplyArgs<double>& a, size_t noe, int k, size_t e, double v, Ld ld,
+                                           double* pnew, double& acc) {
+  constexpr int BASE = apply_base_mode(MODE);
+  const size_t gk = (size_t)k * noe + e;
+  if (BASE == APPLY_RESID) {
+    const double rv = __ldg(a.b + gk) - v;
+    a.out[gk] = rv;
+    acc = fma(rv, rv, acc);
+  } else {
+    a.out[gk] = v;
+    if (BASE == APPLY_CG || BASE == APPLY_DOT) {
+      const double c = ld(k, e);
+      if (BASE == APPLY_CG) pnew[gk] = c;
+      acc = fma(c, v, acc);
+    }
+  }
+}
+
+// The elements x0 + b of row gy for the bits b of todo, by the warp; every
+// ZS-th part of the work for the z-th of the elements' threads.  Returns the
+// lane's share of the reduction.
+//
+// Few elements: one output per lane, as many elements at a time as that fills
+// (the latency of some 4 n FP64 operations each).  Many: one element per lane,
+// its faces' values first; bound by the FP64 pipe.  1024^2, p = 4, and 443^2,
+// p = 8, one element in 1000 uneven (and four neighbours each): 310 and 308 us,
+// none: 264 and 250; all uneven: 1617 and 1571 us (an element per lane alone: the
+// same; an output per lane alone: 3860 and 2706; a kernel of FP64 chains: 1083
+// and 980).
+template <int P, int MODE, int ZS, typename Ld>
+__device__ __noinline__ double chain_elements(const ApplyArgs<double>& a, const Tab<double, P>& tabs, int x0, int gy,
+                                              unsigned todo, int z, Ld ld, double* pnew) {
+  constexpr int N = P, N1 = P + 1, NN = N1 * N1;
+  constexpr bool kPivot = MODE != apply_base_mode(MODE);
+  constexpr int G = NN <= 32 ? 32 / NN : 1;
+  constexpr int kMany = 8 * G > 16 ? 16 : 8 * G;
+  const int lane = threadIdx.x & 31, dim = a.dim;
+  const size_t noe = (size_t)dim * dim;
+  double acc = 0.0;
+  if (__popc(todo) < kMany) {
+    const Tab<double, P>* tb = generic_tab<P>(tabs);
+    const int slot = NN <= 32 ? lane / NN : 0;
+    for (int pick = 0; todo; pick ^= 1) {
+      int gx = -1;  // the slot's element
+#pragma unroll 1
+      for (int g = 0; g < G; ++g, todo &= todo - 1)
+        if (g == slot && todo) gx = x0 + __ffs(todo) - 1;
+      if ((ZS > 1 && pick != z) || gx < 0) continue;
+#pragma unroll 1
+      for (int k = NN <= 32 ? lane % NN : lane; k < NN; k += 32)
+        chain_emit<MODE>(a, noe, k, (size_t)gy * dim + gx,
+                         chain_node<P, kPivot, N1>(tb, a.nu, dim, gx, gy, k / N1, k % N1, ld), ld, pnew, acc);
+    }
+    return acc;
+  }
+  if (!(todo >> lane & 1)) return acc;
+  const int gx = x0 + lane;
+  const size_t e = (size_t)gy * dim + gx;
   double J[4][N1], Q[4][N1];
 #pragma unroll 1
   for (int f = 0; f < 4; ++f) {
-    const bool x = f < 2, zero = (f & 1) == 0;  // zero: this element is the 0 side
-    const bool in = f == 0 ? gx > 0 : (f == 1 ? gx < dim - 1 : (f == 2 ? gy < dim - 1 : gy > 0));
-    const size_t ne = f == 0 ? e - 1 : (f == 1 ? e + 1 : (f == 2 ? e + dim : e - dim));
+    const bool x = f < 2, zero = (f & 1) == 0;
+    size_t ne;
+    const bool in = chain_across(f, dim, gx, gy, e, ne);
 #pragma unroll 1
-    for (int j = 0; j < N1; ++j) {
-      double u0 = 0, d0 = 0, uN = 0, dN = 0;
-      if (zero || in)
-#pragma unroll 1
-        for (int i = 0; i < N1; ++i) {
-          const double v = ld(x ? i * N1 + j : j * N1 + i, zero ? e : ne);
-          if (i == 0) u0 = v;
-          d0 = fma(tb.D0[i], v, d0);
-        }
-      if (!zero || in)
-#pragma unroll 1
-        for (int i = 0; i < N1; ++i) {
-          const double v = ld(x ? i * N1 + j : j * N1 + i, zero ? ne : e);
-          if (i == N) uN = v;
-          dN = fma(tb.DN[i], v, dN);
-        }
-      face_combine<double>(tb.w[j], tb.WH[j], a.nu, in, u0, d0, uN, dN, J[f][j], Q[f][j]);
+    for (int q = 0; q < N1; ++q) {
+      double u0 = 0.0, d0 = 0.0, uN = 0.0, dN = 0.0;
+      if (zero || in) chain_side<P, kPivot, N1>(tabs.D0, x, false, q, zero ? e : ne, ld, u0, d0);
+      if (!zero || in) chain_side<P, kPivot, N1>(tabs.DN, x, true, q, zero ? ne : e, ld, uN, dN);
+      face_combine<double>(tabs.w[q], tabs.WH[q], a.nu, in, u0, d0, uN, dN, J[f][q], Q[f][q]);
     }
   }
-  double acc = 0.0;
 #pragma unroll 1
-  for (int i1 = 0; i1 < N1; ++i1)
+  for (int i1 = z; i1 < N1; i1 += ZS) {
 #pragma unroll 1
     for (int j = 0; j < N1; ++j) {
       double v = face_seed<double, N>(i1, j, Q[0][j], Q[1][j], Q[2][i1], Q[3][i1]);
-      v = fma(tb.D0[i1], J[0][j], fma(tb.DN[i1], J[1][j], v));
-#pragma unroll 1
-      for (int i = 0; i < N1; ++i) v = fma(tb.KW[(i1 * N1 + i) * N1 + j], ld(i * N1 + j, e), v);
-#pragma unroll 1
-      for (int i = 0; i < N1; ++i) v = fma(tb.KW[(j * N1 + i) * N1 + i1], ld(i1 * N1 + i, e), v);
-      v = fma(tb.D0[j], J[2][i1], v);
-      v = fma(tb.DN[j], J[3][i1], v);
-      const size_t gk = (size_t)(i1 * N1 + j) * noe + e;
-      if (BASE == APPLY_RESID) {
-        const double rv = __ldg(a.b + gk) - v;
-        a.out[gk] = rv;
-        acc = fma(rv, rv, acc);
-      } else {
-        a.out[gk] = v;
-        if (kDot) {
-          const double c = ld(i1 * N1 + j, e);
-          if (BASE == APPLY_CG) pnew[gk] = c;
-          acc = fma(c, v, acc);
-        }
-      }
+      v = fma(tabs.D0[i1], J[0][j], fma(tabs.DN[i1], J[1][j], v));
+      v = chain_sum<P, kPivot, N1>(v, [&](int i) { return tabs.KW[(i1 * N1 + i) * N1 + j]; },
+                                   [&](int i) { return ld(i * N1 + j, e); });
+      v = chain_sum<P, kPivot, N1>(v, [&](int i) { return tabs.KW[(j * N1 + i) * N1 + i1]; },
+                                   [&](int i) { return ld(i1 * N1 + i, e); });
+      v = fma(tabs.D0[j], J[2][i1], v);
+      v = fma(tabs.DN[j], J[3][i1], v);
+      chain_emit<MODE>(a, noe, i1 * N1 + j, e, v, ld, pnew, acc);
     }
+  }
   return acc;
 }
 
 // A large penalty's terms into the outputs that this thread (z of ZS) has
-// stored for element (gx, gy); returns its share of the reduction.  (A pass of
-// its own, off the path of the other penalties: as conditions on it, 5 % there.)
+// stored for element (gx, gy); acc: its share of the reduction so far.  (A pass
+// of its own, off the path of the other penalties: as conditions on it, 5 % there.)
 template <int P, int MODE, int ZS, typename Ld>
 __device__ __noinline__ double add_penalty(const ApplyArgs<double>& a, const Tab<double, P>& tb, int gx, int gy, int z,
-                                           Ld ld, const double* pnew) {
+                                           Ld ld, double acc) {
   constexpr int N = P, N1 = P + 1, BASE = apply_base_mode(MODE);
   const size_t noe = (size_t)a.dim * a.dim, e = (size_t)gy * a.dim + gx;
-  double acc = 0.0;
+  auto mine = [&](int i1) { return ZS == 1 || min(i1, N - i1) % ZS == z; };  // the columns it stored
 #pragma unroll 1
-  for (int i1 = 0; i1 < N1; ++i1) {
-    if (ZS > 1 && min(i1, N - i1) % ZS != z) continue;  // its columns
+  for (int f = 0; f < 4; ++f) {
+    const bool x = f < 2, zero = (f & 1) == 0;
+    size_t ne;
+    const bool in = chain_across(f, a.dim, gx, gy, e, ne);
+    double own[N1], other[N1], v[N1];
+#pragma unroll
+    for (int q = 0; q < N1; ++q) {
+      if (!mine(x ? 0 : q)) continue;
+      const int k0 = x ? q : q * N1, kN = x ? N * N1 + q : q * N1 + N;
+      own[q] = ld(zero ? k0 : kN, e);
+      other[q] = in ? ld(zero ? kN : k0, ne) : 0.0;
+      v[q] = a.out[(size_t)(zero ? k0 : kN) * noe + e];
+    }
+#pragma unroll
+    for (int q = 0; q < N1; ++q) {
+      if (!mine(x ? 0 : q)) continue;
+      const int k0 = x ? q : q * N1, kN = x ? N * N1 + q : q * N1 + N;
+      const double t = fx_penalty(tb.w[q], a.nu, own[q], other[q]);
+      a.out[(size_t)(zero ? k0 : kN) * noe + e] = __dadd_rn(v[q], BASE == APPLY_RESID ? -t : t);
+      if (BASE == APPLY_CG || BASE == APPLY_DOT) acc = fma(own[q], t, acc);
+    }
+  }
+  if (BASE == APPLY_RESID) {
+    acc = 0.0;
 #pragma unroll 1
-    for (int j = 0; j < N1; ++j) {
-      const bool face = i1 == 0 || i1 == N || j == 0 || j == N;
-      if (BASE == APPLY_PLAIN && !face) continue;
-      const size_t gk = (size_t)(i1 * N1 + j) * noe + e;
-      double v = a.out[gk];
-      if (face) {
-        const double q = fx_penalty<P>(tb, a.nu, a.dim, gx, gy, i1, j, ld);
-        v = __dadd_rn(v, BASE == APPLY_RESID ? -q : q);
-        a.out[gk] = v;
+    for (int i1 = 0; i1 < N1; ++i1) {
+      if (!mine(i1)) continue;
+#pragma unroll
+      for (int j = 0; j < N1; ++j) {
+        const double v = a.out[(size_t)(i1 * N1 + j) * noe + e];
+        acc = fma(v, v, acc);
       }
-      if (BASE == APPLY_RESID) acc = fma(v, v, acc);
-      else if (BASE == APPLY_CG) acc = fma(pnew[gk], v, acc);
-      else if (BASE == APPLY_DOT) acc = fma(ld(i1 * N1 + j, e), v, acc);
     }
   }
   return acc;
@@ -166,6 +289,7 @@ template <int P, int TX, int TY, int MODE>
 __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const ApplyTab<double, P>& tabs, int bx,
                                               int by, int bid, int nblocks) {
   constexpr int N = P, N1 = P + 1, NN = N1 * N1, TE = TX * TY;
+  static_assert(TX == 32, "a warp is a row of elements");
   constexpr int NE = FxTab<P>::NE, NO = FxTab<P>::NO;
   constexpr int BASE = apply_base_mode(MODE);
   // *_PIVOT modes: the sums over differences from the element's first value
@@ -180,12 +304,12 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red_sh[32];
   __shared__ int2 s_nu[NE];                                   // nu HB(b) w_b
-  __shared__ unsigned s_mag[ZS > 1 ? ZS * TE : 1];
   __shared__ int s_be[(TY + 2) * (TX + 2)];                   // the elements' scales, halo ring included
   __shared__ double s_v0[kPivot ? (TY + 2) * (TX + 2) : 1];   // and pivots
   int2* uf = reinterpret_cast<int2*>(smem_raw);  // values (low word, high word), then limb pairs, in place
   long long* rf = reinterpret_cast<long long*>(smem_raw) + NN * TE;
   long long* ht_ = rf + 4 * N1 * RS;  // the halo elements' traces (doubled)
+  unsigned* lines = reinterpret_cast<unsigned*>(rf);  // phase 0, ZS > 1: what the element's threads know of its lines
 
   if (kDot) {
     if (*(volatile int*)&a.st->done) return;  // converged: the launch is a no-op
@@ -210,7 +334,7 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
   const double* __restrict__ pold = par ? a.pbuf1 : a.pbuf0;
   double* __restrict__ pnew = par ? a.pbuf0 : a.pbuf1;
   auto addr = [&](const double* p, int k) { return fx_addr(p, noe, k); };
-  const FxLoad<BASE == APPLY_CG> ld{a.in, pold, noe, beta, first};
+  const FxLoad<BASE == APPLY_CG, false> ld{a.in, pold, noe, beta, first};
   // the slot of x index (i, odd) and y index (j, odd): even indices at their
   // node, odd ones at the mirrored node
   auto at = [&](int i, bool io, int j, bool jo) -> int { return ((io ? N - i : i) * N1 + (jo ? N - j : j)) * TE + t; };
@@ -225,31 +349,62 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
     return hx >= 0 && hx < dim && hy >= 0 && hy < dim;
   };
   const bool large = fx_large_nu(a.nu * fx.wmax, fx.sk);
-  bool bad = false;
-  if (lt < NE) {
-    s_nu[lt] = large ? make_int2(0, 0) : fx_nu(fx.w[lt] * a.nu, fx.sk);
-  }
+  if (lt < NE) s_nu[lt] = large ? make_int2(0, 0) : fx_nu(fx.w[lt] * a.nu, fx.sk);
 
   // ---- phase 0 --------------------------------------------------------------
   // (raw values in registers where they fit, else in the shared column)
-  unsigned mag = 0;
   double rv_[kRegs ? NN : 1];
   auto raw = [&](int k) -> double {
     if (kRegs) return rv_[kRegs ? k : 0];
     const int2 v = uf[k * TE + t];
     return __hiloint2double(v.y, v.x);
   };
-  auto put_raw = [&](int k, double v) {
-    if (kRegs) rv_[kRegs ? k : 0] = v;
-    else uf[k * TE + t] = make_int2(__double2loint(v), __double2hiint(v));
+  // The element's largest magnitude, and the exponent that every node's row (i1
+  // fixed) or column reaches: in the *_PIVOT modes of the differences along the
+  // line, else of the values.
+  unsigned mag = 0, rows = ~0u, low_words = 0;  // rows: the smallest of them
+  unsigned cmax[N1];                            // columns: largest magnitude, or (pivot) ordered high word
+  int cmin[kPivot ? N1 : 1];
+#pragma unroll
+  for (int j = 0; j < N1; ++j) {
+    cmax[j] = kPivot ? 0x80000000u : 0u;
+    if (kPivot) cmin[j] = 0x7fffffff;
+  }
+  auto row = [&](auto value) {  // value(j): one row
+    unsigned rmax = 0;
+    int rlo = 0x7fffffff, rhi = (int)0x80000000;
+#pragma unroll
+    for (int j = 0; j < N1; ++j) {
+      const double v = value(j);
+      low_words |= (unsigned)__double2loint(v);
+      if (kPivot) {
+        const int o = fx_ordered(__double2hiint(v));
+        rlo = min(rlo, o), rhi = max(rhi, o);
+        cmin[kPivot ? j : 0] = min(cmin[kPivot ? j : 0], o), cmax[j] = (unsigned)max((int)cmax[j], o);
+      } else {
+        const unsigned m = fx_mag(v);
+        rmax = max(rmax, m);
+        cmax[j] = max(cmax[j], m);
+      }
+    }
+    rows = min(rows, kPivot ? fx_apart(rlo, rhi) : rmax);
   };
   const double pv = kPivot && act ? ld(0, e) : 0.0;
-  if constexpr (ZS == 1) {
-#pragma unroll(FxForm<P>::load_unroll)
-    for (int k = 0; k < NN; ++k) put_raw(k, act ? ld(k, e) : 0.0);
+  auto load = [&](int k) {
+    const double v = act ? ld(k, e) : 0.0;
+    return kPivot ? __dadd_rn(v, -pv) : v;
+  };
+  if constexpr (kRegs) {
+#pragma unroll
+    for (int k = 0; k < NN; ++k) rv_[k] = act ? ld(k, e) : 0.0;
   } else {
-#pragma unroll(FxForm<P>::load_unroll / ZS)
-    for (int k = z; k < NN; k += ZS) put_raw(k, act ? ld(k, e) : 0.0);
+#pragma unroll(FxForm<P>::row_unroll)
+    for (int i = z; i < N1; i += ZS)
+      row([&](int j) {
+        const double v = load(i * N1 + j);
+        uf[(i * N1 + j) * TE + t] = make_int2(__double2loint(v), __double2hiint(v));
+        return v;
+      });
   }
   // the halo elements: element h to lane h / kWarps of warp h % kWarps
   for (int h = (lt & 31) * kWarps + (lt >> 5); h < kHalo; h += NT) {
@@ -257,41 +412,61 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
     if (!halo_at(h, hx, hy)) continue;
     const size_t he = (size_t)hy * dim + hx;
     const double v0 = kPivot ? ld(0, he) : 0.0;
-    unsigned hm = 0;
+    unsigned hm = 0, hl = 0;
 #pragma unroll(N1)
-    for (int k = 0; k < NN; ++k) hm = max(hm, fx_mag(kPivot ? __dadd_rn(ld(k, he), -v0) : ld(k, he)));
-    bad = bad || (hm >> 21) >= (unsigned)kFxMaxExp;
-    if ((hm >> 21) < (unsigned)kFxMinExp) {
-      for (int k = 0; k < NN; ++k) bad = bad || (kPivot ? __dadd_rn(ld(k, he), -v0) : ld(k, he)) != 0.0;
+    for (int k = 0; k < NN; ++k) {
+      const double v = kPivot ? __dadd_rn(ld(k, he), -v0) : ld(k, he);
+      hm = max(hm, fx_mag(v));
+      hl |= (unsigned)__double2loint(v);
     }
-    Be(hy - y0, hx - x0) = fx_be(hm);
+    Be(hy - y0, hx - x0) = fx_be(hm, (hm | hl) != 0);
     if (kPivot) V0(hy - y0, hx - x0) = v0;
   }
-#pragma unroll(kRegs ? NN : N1)
-  for (int k = z; k < NN; k += ZS) {
-    if (kPivot) put_raw(k, __dadd_rn(raw(k), -pv));
-    mag = max(mag, fx_mag(raw(k)));
-  }
-  // out of the fixed-point range: this tile takes the plain code (a value
-  // below kFxMinExp only where the whole element is)
-  bool small = false;
-  if ((mag >> 21) < (unsigned)kFxMinExp) {
-#pragma unroll(kRegs ? NN : 1)
-    for (int k = z; k < NN; k += ZS) small = small || raw(k) != 0.0;
+  if constexpr (kRegs) {
+#pragma unroll
+    for (int i = 0; i < N1; ++i)
+      row([&](int j) {
+        double& v = rv_[kRegs ? i * N1 + j : 0];
+        if (kPivot) v = __dadd_rn(v, -pv);
+        return v;
+      });
   }
   if constexpr (ZS > 1) {
-    s_mag[lt] = mag;
-    __syncthreads();  // the other threads' values, and their magnitude
-    mag = max(mag, s_mag[lt ^ TE]);
     static_assert(ZS == 2, "one other thread");
+    auto mine = [&](int q, int tt) -> unsigned& { return lines[q * NT + tt]; };
+#pragma unroll
+    for (int j = 0; j < N1; ++j) {
+      mine(j, lt) = cmax[j];
+      if (kPivot) mine(N1 + 2 + j, lt) = (unsigned)cmin[kPivot ? j : 0];
+    }
+    mine(N1, lt) = rows;
+    mine(N1 + 1, lt) = low_words;
+    __syncthreads();  // the other thread's rows
+    const int other = z ? lt - TE : lt + TE;
+#pragma unroll
+    for (int j = 0; j < N1; ++j) {
+      cmax[j] = kPivot ? (unsigned)max((int)cmax[j], (int)mine(j, other)) : max(cmax[j], mine(j, other));
+      if (kPivot) cmin[kPivot ? j : 0] = min(cmin[kPivot ? j : 0], (int)mine(N1 + 2 + j, other));
+    }
+    rows = min(rows, mine(N1, other));
+    low_words |= mine(N1 + 1, other);
   }
-  bad = bad || (mag >> 21) >= (unsigned)kFxMaxExp || (small && (mag >> 21) < (unsigned)kFxMinExp);
-  const int bs = fx_be(mag);
+  unsigned cols = ~0u;
+#pragma unroll
+  for (int j = 0; j < N1; ++j) {
+    if (kPivot) {
+      const int lo = cmin[kPivot ? j : 0], hi = (int)cmax[j];
+      cols = min(cols, fx_apart(lo, hi));
+      mag = max(mag, max((unsigned)fx_ordered(lo) << 1, (unsigned)fx_ordered(hi) << 1));
+    } else {
+      cols = min(cols, cmax[j]);
+      mag = max(mag, cmax[j]);
+    }
+  }
+  const int low = (int)(max(rows, cols) >> 21);
+  const int bs = fx_be(mag, (mag | low_words) != 0);
   Be(ty, tx) = bs;
-  if (kPivot) {
-    V0(ty, tx) = pv;
-    bad = bad || (fx_mag(pv) >> 21) >= (unsigned)kFxMaxExp;
-  }
+  if (kPivot) V0(ty, tx) = pv;
 #pragma unroll
   for (int i = 0; i < NE; ++i)
 #pragma unroll
@@ -310,10 +485,7 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
       if (!mi && !mj) uf[at(i, true, j, true)] = fx_limbs_of(q[3]);
     }
   double acc = 0.0;
-  const bool plain = __syncthreads_or(bad);
-  if (plain) {
-    if (act && z == 0) acc = plain_element<P, MODE>(a, tabs.t, gx, gy, ld, pnew);
-  } else {
+  __syncthreads();
 
   // ---- phase 1 --------------------------------------------------------------
   // w times the normal derivatives of the element's four faces, component b of
@@ -451,14 +623,19 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
     };
     auto scale = [&](bool in, int row, int col) {
       const int b = in ? max(bs, Be(row, col)) : bs;
-      return kPivot ? max(b, fx_biased(delta(true, ty, tx, in, row, col))) : b;
+      if (!kPivot) return b;
+      const double d = delta(true, ty, tx, in, row, col);
+      return max(b, d != 0.0 && fx_biased(d) <= kFxMinExp ? kFxNoScale : fx_biased(d));
     };
     const Face fl{&R(1, 0, tx > 0 ? t - 1 : TE + ty), &R(0, 0, t), scale(gx > 0, ty, tx - 1)};
     const Face fr{&R(1, 0, t), &R(0, 0, tx < TX - 1 ? t + 1 : TE + ty), scale(gx < dim - 1, ty, tx + 1)};
     const Face fd{&R(3, 0, ty < TY - 1 ? t + TX : TE + tx), &R(2, 0, t), scale(gy < dim - 1, ty + 1, tx)};
     const Face fu{&R(3, 0, t), &R(2, 0, ty > 0 ? t - TX : TE + tx), scale(gy > 0, ty - 1, tx)};
     // the outputs' scale; where it is not the element's own, its values move to it
-    const int be = max(bs, max(max(fl.be, fr.be), max(fd.be, fu.be)) - (kPivot ? 1 : kFxRoom));
+    const int faces = max(max(fl.be, fr.be), max(fd.be, fu.be));
+    const int be = max(bs, faces - (kPivot ? 1 : kFxRoom));
+    const bool fits = act && !fx_chains(be, faces, low);  // one scale fits the element
+    const unsigned todo = __ballot_sync(0xffffffffu, act && !fits);
     if (be > bs)
       for (int k = z; k < NN; k += ZS) uf[k * TE + t] = fx_shift(uf[k * TE + t], min(be - bs, 63));
     if (ZS > 1) __syncthreads();
@@ -582,12 +759,14 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
     };
 #pragma unroll(FxForm<P>::col_unroll)
     for (int i = z; i < NO; i += ZS)
-      if (act) columns(i, std::false_type{});
+      if (fits) columns(i, std::false_type{});
     if constexpr (NE > NO)
-      if (act && z == NO % ZS) columns(NE - 1, std::true_type{});
+      if (fits && z == NO % ZS) columns(NE - 1, std::true_type{});
+    if (large && fits) acc = add_penalty<P, MODE, ZS>(a, tabs.t, gx, gy, z, ld, acc);
+
+    // ---- phase 3 ------------------------------------------------------------
+    if (todo) acc += chain_elements<P, MODE, ZS>(a, tabs.t, x0, gy, todo, z, ld, pnew);
   }
-    if (large && act) acc = add_penalty<P, MODE, ZS>(a, tabs.t, gx, gy, z, ld, pnew);
-  }  // !plain
   if (BASE != APPLY_PLAIN) {
     const double bt = block_sum<double, NT>(acc, red_sh);
     double total;

@@ -28,7 +28,8 @@
 //   5  one output node per thread, then the epilogue (store, direction store
 //      in the CG mode, deterministic grid reduction in the CG / DOT / residual
 //      modes).
-// A tile with values out of the fixed-point range takes the plain FP64 code.
+// An element that one scale does not fit (sipg_fx.cuh) takes FP64 chains in
+// phase 5, its nodes' threads one each.
 #pragma once
 
 #include <algorithm>
@@ -43,6 +44,11 @@ struct PernodeShape {
   static constexpr int N1 = P + 1, NN = N1 * N1;
   static constexpr int EX = pernode_ex(P, SHAPE), EY = pernode_ey(P), NE = EX * EY;
   static constexpr int NT = (NE * NN + 31) / 32 * 32;  // threads: whole warps, the tail idle in phase 2
+  // resident CTAs the registers are limited for: what 80 to 128 a thread allow,
+  // two up to 512 threads (128^2, p = 1, at 128 registers: 10.3 us, at 80: 8.2;
+  // p = 4, shape 1: 45 us with one CTA, 29 with two; p = 6: 53 and 39)
+  static constexpr int MIN_BLOCKS =
+      NT >= 512 ? 1 : (NT > 256 ? 2 : 65536 / (NT * (P == 1 ? 80 : 128)));
   static constexpr int SX = EX + 2, SY = EY + 2;       // element slots, halo ring included
   static constexpr int NX = EY * (EX + 1) * N1;        // x-face nodes: [EY][EX+1][N1]
   static constexpr int NY = EX * (EY + 1) * N1;        // y-face nodes: [EY+1][EX][N1]
@@ -60,6 +66,7 @@ struct PernodeFxSmem {
   long long xj[S::NX], xq[S::NX], yj[S::NY], yq[S::NY];
   long long tot[S::NE * S::NN];  // the output's parity components
   unsigned mag[NSLOT];           // zero between tiles
+  unsigned lines[2 * S::NE];     // the smallest of an element's rows' and columns' largest magnitudes
   int be[NSLOT], bo[S::NE];      // scales of the slots' values, of the outputs
   int xbe[S::EY * (S::EX + 1)], ybe[S::EX * (S::EY + 1)];  // of the faces
   FxTab<P> fx;
@@ -83,6 +90,14 @@ __device__ __forceinline__ void pernode_fx_tables(PernodeFxSmem<P, SHAPE>& sm, c
   }
   if (t == 0) sm.large = large;
   __syncthreads();
+}
+
+// (Three terms in flight: with all of them the call's registers cost every
+// per-node tile; 128^2, p = 5: 34 us instead of 29.)
+template <int P, typename Ld>
+__device__ __noinline__ double chain_node_call(const Tab<double, P>& tabs, double nu, int dim, int gx, int gy, int i1,
+                                               int j, Ld ld) {
+  return chain_node<P, false, 3>(generic_tab<P>(tabs), nu, dim, gx, gy, i1, j, ld);
 }
 
 // One tile (origin x0, y0): phases 0-5, returning this thread's share of the
@@ -116,6 +131,7 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
   };
   // ---- phase 0: values and magnitudes ----------------------------------------
   // (every load of the thread first, so that they are in flight together)
+  if (t < 2 * NE) sm.lines[t] = ~0u;
   constexpr int IT = (NSLOT * NN + NT - 1) / NT;
   double vr[IT], vp[IT];
 #pragma unroll
@@ -135,30 +151,22 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
     const int sy = sl / SX, sx = sl - sy * SX;
     if (idx >= NSLOT * NN) break;
     const double v = MODE == APPLY_CG && !first ? fma(beta, vp[it], vr[it]) : vr[it];
-    if (fx_mag(v) != 0) atomicMax(&sm.mag[sl], fx_mag(v));
+    const unsigned m = fx_mag(v) | min((unsigned)__double2loint(v), 1u);  // zero for zeros only
+    if (m != 0) atomicMax(&sm.mag[sl], m);
     sm.us[sl * NN + k] = make_int2(__double2loint(v), __double2hiint(v));
     if (sx > 0 && sx < SX - 1 && sy > 0 && sy < SY - 1) sm.own[k * NE + (sy - 1) * EX + sx - 1] = v;
   }
   __syncthreads();
   // ---- phase 1: parity form ---------------------------------------------------
-  bool bad = false;
-  for (int sl = t; sl < NSLOT; sl += NT) {
-    const unsigned b = sm.mag[sl] >> 21;
-    bad = bad || b >= (unsigned)kFxMaxExp;
-    if (b < (unsigned)kFxMinExp && b > 0) bad = true;  // (b = 0: zeros and denormals, told apart below)
-    sm.be[sl] = fx_be(sm.mag[sl]);
-  }
+  auto scale = [&](int sl) { return fx_be(sm.mag[sl], sm.mag[sl] != 0); };
+  for (int sl = t; sl < NSLOT; sl += NT) sm.be[sl] = scale(sl);
   for (int task = t; task < NSLOT * HE * HE; task += NT) {
     const int sl = task / (HE * HE), q2 = task - sl * (HE * HE), i = q2 / HE, j = q2 - i * HE;
-    const int be = fx_be(sm.mag[sl]);
+    const int be = scale(sl);
     const bool mi = 2 * i == N, mj = 2 * j == N;
     int2* u = sm.us + sl * NN;
     const int k0 = i * N1 + j, k1 = (N - i) * N1 + j, k2 = i * N1 + N - j, k3 = (N - i) * N1 + N - j;
-    auto raw = [&](int k) {
-      const double v = __hiloint2double(u[k].y, u[k].x);
-      bad = bad || (fx_biased(v) == 0 && v != 0.0 && be == kFxMinExp);
-      return v;
-    };
+    auto raw = [&](int k) { return __hiloint2double(u[k].y, u[k].x); };
     long long q[4];
     q[0] = fx_fix(raw(k0), be);
     q[1] = mi ? 0 : fx_fix(raw(k1), be);
@@ -170,14 +178,7 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
     if (!mj) u[k2] = fx_limbs_of(q[2]);
     if (!mi && !mj) u[k3] = fx_limbs_of(q[3]);
   }
-  if (__syncthreads_or(bad)) {  // out of the fixed-point range: the plain code, one element per thread
-    double r = 0.0;
-    if (t < NE && x0 + t % EX < dim && y0 + t / EX < dim)
-      r = plain_element<P, MODE>(a, tabs.t, x0 + t % EX, y0 + t / EX, ld, pnew);
-    for (int sl = t; sl < NSLOT; sl += NT) sm.mag[sl] = 0;
-    __syncthreads();
-    return r;
-  }
+  __syncthreads();
   // ---- phase 2: normal derivatives -------------------------------------------
   constexpr int TX_ = EY * SX * N1, TY_ = SY * EX * N1;
   for (int task = t; task < TX_ + TY_; task += NT) {
@@ -236,6 +237,7 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
   }
   __syncthreads();
   // ---- phase 4: the output's parity components -----------------------------------
+  int be_out = 0, faces = 0;  // the scales of the thread's element
   if (t < NE * NN) {
     const int le = t % NE, k = t / NE, ex = le % EX, ey = le / EX;
     const int ka = k / N1, kb = k - ka * N1;  // slot indices along x and y
@@ -245,7 +247,18 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
       const int bs = sm.be[sl];
       const int fL = ey * (EX + 1) + ex, fR = fL + 1, fU = ey * EX + ex, fD = fU + EX;  // faces
       const int bL = sm.xbe[fL], bR = sm.xbe[fR], bU = sm.ybe[fU], bD = sm.ybe[fD];
-      const int be = max(bs, max(max(bL, bR), max(bD, bU)) - kFxRoom);
+      faces = max(max(bL, bR), max(bD, bU));
+      const int be = be_out = max(bs, faces - kFxRoom);
+      if (k < N1) {  // one row and one column each
+        unsigned row = 0, col = 0;
+#pragma unroll
+        for (int i = 0; i < N1; ++i) {
+          row = max(row, fx_mag(sm.own[(i * N1 + k) * NE + le]));
+          col = max(col, fx_mag(sm.own[(k * N1 + i) * NE + le]));
+        }
+        atomicMin(&sm.lines[2 * le], row);
+        atomicMin(&sm.lines[2 * le + 1], col);
+      }
       const int so = be - bs, xp = fx_exp(be, fx.sk);
       auto own = [&](int kk) { return so > 0 ? fx_shift(u[kk], min(so, 63)) : u[kk]; };
       const bool oa = ka >= HE, ob = kb >= HE;  // odd indices sit at the mirrored slots
@@ -297,8 +310,20 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
       long long r = row(i);
       if (2 * i != N) r = i1 == i ? r + row(N - i) : r - row(N - i);
       double v = fx_double(r, sm.bo[le]);
-      if (sm.large && (i1 == 0 || i1 == N || j == 0 || j == N))
-        v = __dadd_rn(v, fx_penalty<P>(tabs.t, a.nu, dim, gx, gy, i1, j, ld));
+      if (fx_chains(be_out, faces, (int)(max(sm.lines[2 * le], sm.lines[2 * le + 1]) >> 21))) {
+        v = chain_node_call<P>(tabs.t, a.nu, dim, gx, gy, i1, j,
+                               FxLoad<MODE == APPLY_CG, kCoherent>{a.in, pold, (unsigned)noe, beta, first});
+      } else if (sm.large) {
+        const size_t e = (size_t)gy * dim + gx;
+        const double own = sm.own[k * NE + le];
+        auto face = [&](double w, bool in, int ka, size_t ne) {
+          v = __dadd_rn(v, fx_penalty(w, a.nu, own, in ? ld(ka, ne) : 0.0));
+        };
+        if (i1 == 0) face(tabs.t.w[j], gx > 0, N * N1 + j, e - 1);
+        if (i1 == N) face(tabs.t.w[j], gx < dim - 1, j, e + 1);
+        if (j == 0) face(tabs.t.w[i1], gy < dim - 1, i1 * N1 + N, e + dim);
+        if (j == N) face(tabs.t.w[i1], gy > 0, i1 * N1, e - dim);
+      }
       const size_t gk = (size_t)k * noe + (size_t)gy * dim + gx;
       if (MODE == APPLY_RESID) {
         const double rv = __ldg(a.b + gk) - v;
@@ -317,7 +342,7 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
 }
 
 template <typename T, int P, int SHAPE, int MODE>
-__global__ void __launch_bounds__(PernodeShape<P, SHAPE>::NT)
+__global__ void __launch_bounds__(PernodeShape<P, SHAPE>::NT, PernodeShape<P, SHAPE>::MIN_BLOCKS)
     k_sipg_apply_pernode(const __grid_constant__ ApplyArgs<T> a, const __grid_constant__ ApplyTab<T, P> tb) {
   using S = PernodeShape<P, SHAPE>;
   constexpr int EX = S::EX, EY = S::EY, NT = S::NT;

@@ -28,7 +28,7 @@
 // Large penalties (fx_large_nu).  A jump's integer is rounded at the quantum of
 // the face's larger element, and nu multiplies that; so beyond some tens of
 // units the integer sums leave the penalty out, and it joins the outputs of the
-// face nodes as nu w (u_0side - u_Nside) in FP64 (fx_penalty).  Relative 2-norm
+// face nodes as nu w (u - u_across) in FP64 (fx_penalty).  Relative 2-norm
 // error on sin(2 pi x) sin(3 pi y), 12^2 elements, p = 4, penalty 100 p^2: 9.0e-14
 // with integer jumps, 1.4e-14 with FP64 ones, 1.8e-14 with FP64 chains.
 //
@@ -39,10 +39,24 @@
 // derivative) sum to zero exactly.  An element whose neighbour is more than
 // 2^kFxRoom times larger takes a coarser scale.
 //
+// That is accuracy relative to the element's (and its neighbours') largest
+// values.  An output sums its own row and column of the element, its face terms
+// and the traces across, and where those are all small, chains keep it accurate
+// relative to them and one scale for the element does not.  So the elements
+// that one scale does not fit take FP64 chains instead (chain_node), each by
+// itself: those where some node's row and column both stay below 2^-kFxSpread of
+// the scale, which an element far smaller than a neighbour is too, and zeros
+// beside non-zeros.  The others' entry-wise error is bounded by the scale;
+// against the sum of the entry's terms it reaches 900 2^-53 (a load vector,
+// whose corner nodes carry small weights, p = 8; chains: 4 2^-53), 15 2^-53 on
+// uniform values (chains 13).  CG directions, p = 1..8: 0.1 to 1.2 in 1000
+// elements lie beyond 2^-4, 3 to 30 beyond 2^-2.
+//
 // Range.  The scale is the element's own, so vectors of any magnitude keep
 // this accuracy.  An element with an infinity, a NaN, or a magnitude near the
-// ends of the exponent range (kFxMinExp, kFxMaxExp) sends its tile to the
-// plain FP64 code.
+// ends of the exponent range (kFxMinExp, kFxMaxExp) has no scale: it and its
+// neighbours take the chains.  Which elements do depends on the element and its
+// four neighbours alone.
 #pragma once
 
 #include <cmath>
@@ -55,7 +69,9 @@ namespace sipg {
 constexpr int kFxLimb = 29;                       // bits of a low limb
 constexpr int kFxBits = 55;                       // a value's integer is below 2^kFxBits
 constexpr int kFxRoom = 2;                        // bits a neighbour's scale may exceed the element's
-constexpr int kFxMinExp = 200, kFxMaxExp = 1983;  // biased exponents an element's largest value may have
+constexpr int kFxSpread = 4;                      // bits a node's row and column may both stay below the scale
+constexpr int kFxMinExp = 200, kFxMaxExp = 1983;  // an element's largest value's biased exponent lies between
+constexpr int kFxNoScale = 2047;                  // the scale of an element where it does not
 
 // Fixed-point tables of degree P in parity form (limb pairs, .x = h, .y = l).
 // Mirrored nodes i and N - i have the even index i and the odd index i (< NO);
@@ -259,8 +275,24 @@ __device__ __forceinline__ double fx_double(long long r, int ex) {
 
 // For the running maximum of magnitudes: the high word less its sign.
 __device__ __forceinline__ unsigned fx_mag(double v) { return (unsigned)__double2hiint(v) << 1; }
-// The scale of an element whose largest fx_mag is m.
-__device__ __forceinline__ int fx_be(unsigned m) { return max((int)(m >> 21), kFxMinExp); }
+// The scale of an element whose largest fx_mag is m: kFxMinExp for zeros only.
+__device__ __forceinline__ int fx_be(unsigned m, bool nonzero) {
+  const int e = (int)(m >> 21);
+  if (e >= kFxMaxExp || (e <= kFxMinExp && nonzero)) return kFxNoScale;
+  return max(e, kFxMinExp);
+}
+// Whether an element takes the chains: its outputs' scale be, the largest of its
+// and its faces' scales (faces), and the exponent low that every node's row or
+// column reaches.
+__device__ __forceinline__ bool fx_chains(int be, int faces, int low) {
+  return be >= kFxMaxExp || (low < be - kFxSpread && faces > kFxMinExp);
+}
+// The high word of a double as an integer of the same order, and back.
+__device__ __forceinline__ int fx_ordered(int hi) { return hi ^ ((hi >> 31) & 0x7fffffff); }
+// How far apart two values are whose ordered high words are lo <= hi, as fx_mag.
+__device__ __forceinline__ unsigned fx_apart(int lo, int hi) {
+  return fx_mag(__dadd_rn(__hiloint2double(fx_ordered(hi), 0), -__hiloint2double(fx_ordered(lo), 0)));
+}
 // Twice the trace of an element: its even value of index 0 along the normal plus
 // (0 side) or less (N side) the odd one.
 __device__ __forceinline__ long long fx_trace0(int2 e, int2 o) {
@@ -344,25 +376,11 @@ __device__ __forceinline__ void fx_face(int2 nu, bool in0, bool inN, long long t
   if (!(in0 && inN)) J *= 2;
 }
 
-// The penalty's FP64 term of output (i1, j) of element e = (gx, gy): nu w times
-// the node's value less the value across, summed over the faces the node lies
-// on.  ld(k, element): the operator's input.
-template <int P, typename Ld>
-__device__ __forceinline__ double fx_penalty(const Tab<double, P>& tb, double nu, int dim, int gx, int gy, int i1, int j,
-                                             Ld ld) {
-  constexpr int N = P, N1 = P + 1;
-  const size_t e = (size_t)gy * dim + gx;
-  const double own = ld(i1 * N1 + j, e);
-  double v = 0.0;
-  // (explicitly rounded: the same bits wherever it is inlined)
-  auto face = [&](double w, bool in, int k, size_t ne) {
-    v = __dadd_rn(v, __dmul_rn(__dmul_rn(w, nu), __dadd_rn(own, in ? -ld(k, ne) : 0.0)));
-  };
-  if (i1 == 0) face(tb.w[j], gx > 0, N * N1 + j, e - 1);
-  if (i1 == N) face(tb.w[j], gx < dim - 1, j, e + 1);
-  if (j == 0) face(tb.w[i1], gy < dim - 1, i1 * N1 + N, e + dim);
-  if (j == N) face(tb.w[i1], gy > 0, i1 * N1, e - dim);
-  return v;
+// A large penalty's FP64 term of an output on a face: nu w times the node's
+// value less the value across.  (Explicitly rounded: the same bits wherever it
+// is inlined.)
+__device__ __forceinline__ double fx_penalty(double w, double nu, double own, double across) {
+  return __dmul_rn(__dmul_rn(w, nu), __dadd_rn(own, -across));
 }
 
 }  // namespace sipg

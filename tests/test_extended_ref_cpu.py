@@ -23,4 +23,5 @@ def test_extended_reference_matches_the_oracle(oracle):
     for p, dim in ((1, 3), (3, 2), (8, 4)):
         x = rng.uniform(-1, 1, dim * dim * (p + 1) ** 2)
         ref, S = ext.apply(dim, p, 7.0 * p, x)
+        assert np.max(np.abs(ext.apply(dim, p, 7.0 * p, x, pivot=True)[0] - ref) / S) <= 1e-17
         assert np.max(np.abs(oracle.apply(p, dim, 7.0 * p, x) - ref) / S) <= (2 * p + 8) * 2.0 ** -53
