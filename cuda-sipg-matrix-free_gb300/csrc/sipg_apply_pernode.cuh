@@ -386,22 +386,25 @@ __global__ void __launch_bounds__(PernodeShape<P, SHAPE>::NT, PernodeShape<P, SH
 }
 
 // Resident CTAs of a per-node kernel on the current device (occupancy x SMs),
-// computed once per kernel.
-template <typename K>
-int pernode_resident_blocks(K kernel, int threads) {
-  static std::atomic<int> cached{0};
-  int v = cached.load(std::memory_order_relaxed);
-  if (v > 0) return v;
+// computed once per kernel and device.  (The kernel is a template argument: the
+// shapes and modes of a degree share one function type, and a count kept per
+// type was the first one's for all, so that the CTAs of a reduction depended on
+// what had run before.)
+template <auto KERNEL>
+int pernode_resident_blocks(int threads) {
+  constexpr int kDevices = 64;
+  static std::atomic<int> cached[kDevices];
   int dev = 0, sms = 0, per_sm = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess || per_sm < 1) {
+  if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+  const bool keep = dev >= 0 && dev < kDevices;
+  if (keep && cached[dev].load(std::memory_order_relaxed) > 0) return cached[dev].load(std::memory_order_relaxed);
+  if (dev < 0 || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERNEL, threads, 0) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     return 152;  // one CTA per SM of a GB300
   }
-  v = sms * per_sm;
-  cached.store(v, std::memory_order_relaxed);
-  return v;
+  if (keep) cached[dev].store(sms * per_sm, std::memory_order_relaxed);
+  return sms * per_sm;
 }
 
 template <typename T, int P, int SHAPE>
@@ -412,35 +415,22 @@ cudaError_t launch_apply_pernode_shape(int mode, const ApplyArgs<T>& a, const Ap
   const long long ntiles = (long long)((a.dim + S::EX - 1) / S::EX) * ((rows + S::EY - 1) / S::EY);
   // at most the resident CTAs, and in a reducing mode at most one partial per
   // scratch entry
-  auto grid_for = [&](auto kernel, bool reduces) {
-    long long g = std::min<long long>(ntiles, pernode_resident_blocks(kernel, S::NT));
+  auto grid_for = [&](int resident, bool reduces) {
+    long long g = std::min<long long>(ntiles, resident);
     if (reduces) g = std::min<long long>(g, a.red.capacity);
     return (int)std::max<long long>(g, 1);
   };
-  const dim3 block(S::NT);
+  auto launch = [&](auto mode_c) {
+    constexpr int MODE = decltype(mode_c)::value;
+    constexpr auto kernel = k_sipg_apply_pernode<T, P, SHAPE, MODE>;
+    kernel<<<grid_for(pernode_resident_blocks<kernel>(S::NT), MODE != APPLY_PLAIN), dim3(S::NT), 0, s>>>(a, tb);
+  };
   switch (mode) {
-    case APPLY_PLAIN: {
-      auto k = k_sipg_apply_pernode<T, P, SHAPE, APPLY_PLAIN>;
-      k<<<grid_for(k, false), block, 0, s>>>(a, tb);
-      break;
-    }
-    case APPLY_CG: {
-      auto k = k_sipg_apply_pernode<T, P, SHAPE, APPLY_CG>;
-      k<<<grid_for(k, true), block, 0, s>>>(a, tb);
-      break;
-    }
-    case APPLY_RESID: {
-      auto k = k_sipg_apply_pernode<T, P, SHAPE, APPLY_RESID>;
-      k<<<grid_for(k, true), block, 0, s>>>(a, tb);
-      break;
-    }
-    case APPLY_DOT: {
-      auto k = k_sipg_apply_pernode<T, P, SHAPE, APPLY_DOT>;
-      k<<<grid_for(k, true), block, 0, s>>>(a, tb);
-      break;
-    }
-    default:
-      return cudaErrorInvalidValue;
+    case APPLY_PLAIN: launch(std::integral_constant<int, APPLY_PLAIN>{}); break;
+    case APPLY_CG: launch(std::integral_constant<int, APPLY_CG>{}); break;
+    case APPLY_RESID: launch(std::integral_constant<int, APPLY_RESID>{}); break;
+    case APPLY_DOT: launch(std::integral_constant<int, APPLY_DOT>{}); break;
+    default: return cudaErrorInvalidValue;
   }
   count_launch();
   return cudaGetLastError();
