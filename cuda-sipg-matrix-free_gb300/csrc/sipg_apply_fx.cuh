@@ -242,8 +242,8 @@ __device__ __noinline__ double chain_elements(const ApplyArgs<double>& a, const 
 // stored for element (gx, gy); acc: its share of the reduction so far.  (A pass
 // of its own, off the path of the other penalties: as conditions on it, 5 % there.)
 template <int P, int MODE, int ZS, typename Ld>
-__device__ __noinline__ double add_penalty(const ApplyArgs<double>& a, const Tab<double, P>& tb, int gx, int gy, int z,
-                                           Ld ld, double acc) {
+__device__ __noinline__ double add_penalty(const ApplyArgs<double>& a, const ApplyTab<double, P>& tabs, int gx, int gy,
+                                           int z, Ld ld, double acc) {
   constexpr int N = P, N1 = P + 1, BASE = apply_base_mode(MODE);
   const size_t noe = (size_t)a.dim * a.dim, e = (size_t)gy * a.dim + gx;
   auto mine = [&](int i1) { return ZS == 1 || min(i1, N - i1) % ZS == z; };  // the columns it stored
@@ -265,7 +265,7 @@ __device__ __noinline__ double add_penalty(const ApplyArgs<double>& a, const Tab
     for (int q = 0; q < N1; ++q) {
       if (!mine(x ? 0 : q)) continue;
       const int k0 = x ? q : q * N1, kN = x ? N * N1 + q : q * N1 + N;
-      const double t = fx_penalty(tb.w[q], a.nu, own[q], other[q]);
+      const double t = fx_penalty(tabs.t.w[q], tabs.fx.wl[q], a.nu, own[q], other[q]);
       a.out[(size_t)(zero ? k0 : kN) * noe + e] = __dadd_rn(v[q], BASE == APPLY_RESID ? -t : t);
       if (BASE == APPLY_CG || BASE == APPLY_DOT) acc = fma(own[q], t, acc);
     }
@@ -762,7 +762,7 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
       if (fits) columns(i, std::false_type{});
     if constexpr (NE > NO)
       if (fits && z == NO % ZS) columns(NE - 1, std::true_type{});
-    if (large && fits) acc = add_penalty<P, MODE, ZS>(a, tabs.t, gx, gy, z, ld, acc);
+    if (large && fits) acc = add_penalty<P, MODE, ZS>(a, tabs, gx, gy, z, ld, acc);
 
     // ---- phase 3 ------------------------------------------------------------
     if (todo) acc += chain_elements<P, MODE, ZS>(a, tabs.t, x0, gy, todo, z, ld, pnew);

@@ -316,13 +316,13 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
       } else if (sm.large) {
         const size_t e = (size_t)gy * dim + gx;
         const double own = sm.own[k * NE + le];
-        auto face = [&](double w, bool in, int ka, size_t ne) {
-          v = __dadd_rn(v, fx_penalty(w, a.nu, own, in ? ld(ka, ne) : 0.0));
+        auto face = [&](int q, bool in, int ka, size_t ne) {
+          v = __dadd_rn(v, fx_penalty(tabs.t.w[q], fx.wl[q], a.nu, own, in ? ld(ka, ne) : 0.0));
         };
-        if (i1 == 0) face(tabs.t.w[j], gx > 0, N * N1 + j, e - 1);
-        if (i1 == N) face(tabs.t.w[j], gx < dim - 1, j, e + 1);
-        if (j == 0) face(tabs.t.w[i1], gy < dim - 1, i1 * N1 + N, e + dim);
-        if (j == N) face(tabs.t.w[i1], gy > 0, i1 * N1, e - dim);
+        if (i1 == 0) face(j, gx > 0, N * N1 + j, e - 1);
+        if (i1 == N) face(j, gx < dim - 1, j, e + 1);
+        if (j == 0) face(i1, gy < dim - 1, i1 * N1 + N, e + dim);
+        if (j == N) face(i1, gy > 0, i1 * N1, e - dim);
       }
       const size_t gk = (size_t)k * noe + (size_t)gy * dim + gx;
       if (MODE == APPLY_RESID) {

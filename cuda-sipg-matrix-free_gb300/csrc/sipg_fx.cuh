@@ -87,7 +87,8 @@ struct FxTab {
   // lift: times J_0side -+ J_Nside.  As a derivative: HB w_b times the 0 side's
   // is twice (even + odd), HB w_b times the N side's twice (odd - even).
   int2 le[NE * NE], lo[NO * NE];
-  double w[NE];  // HB(b) w_b, and the largest
+  double wl[N1];  // the weights beyond Tab::w
+  double w[NE];   // HB(b) w_b, and the largest
   double wmax;
   int sk;  // coefficient = F 2^-sk
 };
@@ -217,6 +218,7 @@ inline FxTab<P> make_fxtab(const HostTables& h) {
     t.w[i] = (double)hw(i);
     t.wmax = std::fmax(t.wmax, t.w[i]);
   }
+  for (int i = 0; i < n; ++i) t.wl[i] = (double)(w[i] - (long double)h.w[i]);
   return t;
 }
 
@@ -377,10 +379,15 @@ __device__ __forceinline__ void fx_face(int2 nu, bool in0, bool inN, long long t
 }
 
 // A large penalty's FP64 term of an output on a face: nu w times the node's
-// value less the value across.  (Explicitly rounded: the same bits wherever it
-// is inlined.)
-__device__ __forceinline__ double fx_penalty(double w, double nu, double own, double across) {
-  return __dmul_rn(__dmul_rn(w, nu), __dadd_rn(own, -across));
+// value less the value across, w = wh + wl.  The coefficient is carried in two
+// doubles: rounded to one, its error is the same at every node of a line and
+// does not average out (uniform values, p = 6, 100 p^2: 2-norm error 1.0 2^-52 of
+// the terms, here 0.5).  (Explicitly rounded: the same bits wherever it is
+// inlined.)
+__device__ __forceinline__ double fx_penalty(double wh, double wl, double nu, double own, double across) {
+  const double jump = __dadd_rn(own, -across), c = __dmul_rn(wh, nu);
+  const double cl = __fma_rn(wl, nu, __fma_rn(wh, nu, -c));
+  return __fma_rn(c, jump, __dmul_rn(cl, jump));
 }
 
 }  // namespace sipg
