@@ -239,11 +239,12 @@ __device__ __noinline__ double chain_elements(const ApplyArgs<double>& a, const 
 }
 
 // A large penalty's terms into the outputs that this thread (z of ZS) has
-// stored for element (gx, gy); acc: its share of the reduction so far.  (A pass
+// stored for element (gx, gy), pen[q] the coefficient at node q of a face; acc:
+// its share of the reduction so far.  (A pass
 // of its own, off the path of the other penalties: as conditions on it, 5 % there.)
 template <int P, int MODE, int ZS, typename Ld>
-__device__ __noinline__ double add_penalty(const ApplyArgs<double>& a, const ApplyTab<double, P>& tabs, int gx, int gy,
-                                           int z, Ld ld, double acc) {
+__device__ __noinline__ double add_penalty(const ApplyArgs<double>& a, const double2* pen, int gx, int gy, int z, Ld ld,
+                                           double acc) {
   constexpr int N = P, N1 = P + 1, BASE = apply_base_mode(MODE);
   const size_t noe = (size_t)a.dim * a.dim, e = (size_t)gy * a.dim + gx;
   auto mine = [&](int i1) { return ZS == 1 || min(i1, N - i1) % ZS == z; };  // the columns it stored
@@ -265,9 +266,10 @@ __device__ __noinline__ double add_penalty(const ApplyArgs<double>& a, const App
     for (int q = 0; q < N1; ++q) {
       if (!mine(x ? 0 : q)) continue;
       const int k0 = x ? q : q * N1, kN = x ? N * N1 + q : q * N1 + N;
-      const double t = fx_penalty(tabs.t.w[q], tabs.fx.wl[q], a.nu, own[q], other[q]);
-      a.out[(size_t)(zero ? k0 : kN) * noe + e] = __dadd_rn(v[q], BASE == APPLY_RESID ? -t : t);
-      if (BASE == APPLY_CG || BASE == APPLY_DOT) acc = fma(own[q], t, acc);
+      const double2 c = pen[q];
+      const double jump = BASE == APPLY_RESID ? __dadd_rn(other[q], -own[q]) : __dadd_rn(own[q], -other[q]);
+      a.out[(size_t)(zero ? k0 : kN) * noe + e] = fx_add_penalty(v[q], c, jump);
+      if (BASE == APPLY_CG || BASE == APPLY_DOT) acc = fma(own[q], fma(c.x, jump, c.y * jump), acc);
     }
   }
   if (BASE == APPLY_RESID) {
@@ -304,6 +306,7 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red_sh[32];
   __shared__ int2 s_nu[NE];                                   // nu HB(b) w_b
+  __shared__ double2 s_pen[N1];                               // nu w, if large
   __shared__ int s_be[(TY + 2) * (TX + 2)];                   // the elements' scales, halo ring included
   __shared__ double s_v0[kPivot ? (TY + 2) * (TX + 2) : 1];   // and pivots
   int2* uf = reinterpret_cast<int2*>(smem_raw);  // values (low word, high word), then limb pairs, in place
@@ -349,6 +352,7 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
     return hx >= 0 && hx < dim && hy >= 0 && hy < dim;
   };
   const bool large = fx_large_nu(a.nu * fx.wmax, fx.sk);
+  if (large && lt < N1) s_pen[lt] = fx_penalty(tabs.t.w[lt], fx.wl[lt], a.nu);
   if (lt < NE) s_nu[lt] = large ? make_int2(0, 0) : fx_nu(fx.w[lt] * a.nu, fx.sk);
 
   // ---- phase 0 --------------------------------------------------------------
@@ -762,7 +766,7 @@ __device__ __forceinline__ void apply_tile_fx(const ApplyArgs<double>& a, const 
       if (fits) columns(i, std::false_type{});
     if constexpr (NE > NO)
       if (fits && z == NO % ZS) columns(NE - 1, std::true_type{});
-    if (large && fits) acc = add_penalty<P, MODE, ZS>(a, tabs, gx, gy, z, ld, acc);
+    if (large && fits) acc = add_penalty<P, MODE, ZS>(a, s_pen, gx, gy, z, ld, acc);
 
     // ---- phase 3 ------------------------------------------------------------
     if (todo) acc += chain_elements<P, MODE, ZS>(a, tabs.t, x0, gy, todo, z, ld, pnew);

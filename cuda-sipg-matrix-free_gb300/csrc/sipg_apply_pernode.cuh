@@ -317,7 +317,7 @@ __device__ __forceinline__ double pernode_tile_fx(const ApplyArgs<double>& a, Pe
         const size_t e = (size_t)gy * dim + gx;
         const double own = sm.own[k * NE + le];
         auto face = [&](int q, bool in, int ka, size_t ne) {
-          v = __dadd_rn(v, fx_penalty(tabs.t.w[q], fx.wl[q], a.nu, own, in ? ld(ka, ne) : 0.0));
+          v = fx_add_penalty(v, fx_penalty(tabs.t.w[q], fx.wl[q], a.nu), __dadd_rn(own, in ? -ld(ka, ne) : 0.0));
         };
         if (i1 == 0) face(j, gx > 0, N * N1 + j, e - 1);
         if (i1 == N) face(j, gx < dim - 1, j, e + 1);

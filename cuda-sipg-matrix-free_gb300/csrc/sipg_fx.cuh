@@ -378,16 +378,18 @@ __device__ __forceinline__ void fx_face(int2 nu, bool in0, bool inN, long long t
   if (!(in0 && inN)) J *= 2;
 }
 
-// A large penalty's FP64 term of an output on a face: nu w times the node's
-// value less the value across, w = wh + wl.  The coefficient is carried in two
-// doubles: rounded to one, its error is the same at every node of a line and
-// does not average out (uniform values, p = 6, 100 p^2: 2-norm error 1.0 2^-52 of
-// the terms, here 0.5).  (Explicitly rounded: the same bits wherever it is
+// A large penalty's coefficient nu w, w = wh + wl, in two doubles: rounded to
+// one, its error is the same at every node of a line and does not average out
+// (uniform values, p = 6, 100 p^2: 2-norm error 1.0 2^-52 of the terms, here
+// 0.5).  And its FP64 term added to an output v on a face, whose value exceeds the
+// one across by jump.  (Explicitly rounded: the same bits wherever they are
 // inlined.)
-__device__ __forceinline__ double fx_penalty(double wh, double wl, double nu, double own, double across) {
-  const double jump = __dadd_rn(own, -across), c = __dmul_rn(wh, nu);
-  const double cl = __fma_rn(wl, nu, __fma_rn(wh, nu, -c));
-  return __fma_rn(c, jump, __dmul_rn(cl, jump));
+__device__ __forceinline__ double2 fx_penalty(double wh, double wl, double nu) {
+  const double c = __dmul_rn(wh, nu);
+  return make_double2(c, __fma_rn(wl, nu, __fma_rn(wh, nu, -c)));
+}
+__device__ __forceinline__ double fx_add_penalty(double v, double2 c, double jump) {
+  return __fma_rn(c.x, jump, __fma_rn(c.y, jump, v));
 }
 
 }  // namespace sipg
