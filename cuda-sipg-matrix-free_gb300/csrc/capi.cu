@@ -141,8 +141,8 @@ static TileCfg default_cfg(int p, int dim, bool f64) {
   c.tx = 32;
   if (f64) {
     // 32 x TY tiles by measurement at ~16 M DoF (us with 2, 4, 8 rows): p = 1:
-    // 259, 199, 197; 2: 238, 172, 164; 3: 239, 178, 170; 4 (1024^2): 414, 285,
-    // 267; 5: 277, 202, 253; 6: 269, 228, 250; 7: 261, 240, 264; 8: 291, 353, too
+    // 253, 193, 189; 2: 213, 162, 154; 3: 201, 162, 156; 4 (1024^2): 375, 273,
+    // 262; 5: 245, 185, 235; 6: 243, 207, 231; 7: 237, 218, 245; 8: 249, 287, too
     // large
     static const int kRows[9] = {4, 8, 8, 8, 8, 4, 4, 4, 2};
     c.ty = kRows[p >= 1 && p <= 8 ? p : 0];
@@ -249,7 +249,8 @@ static int graph_iters(long long ndof) { return ndof <= (1LL << 20) ? 32 : 8; }
 // (APPLY_CG: two kernels per iteration).  The per-node tile does: on the small
 // meshes it serves, an iteration is a chain of short launches.  The
 // element-per-thread tiles form the direction in a vector kernel instead
-// (APPLY_DOT), so the apply reads one vector, not two.
+// (APPLY_DOT), so the apply reads one vector, not two (decided with FP64 chains in
+// the apply, whose FP64 pipe the direction's operations would have shared).
 template <typename T>
 static bool cg_fused_direction(const sipg_op* op) {
   return sizeof(T) == 8 && is_pernode(op->cfg64, op->p);
@@ -338,7 +339,7 @@ static sipg_status cg_solve(sipg_op* op, T* x, const T* b, T tol, int rel, int m
   const int K = graph_iters(op->ndof);
   // small FP64 meshes on the per-node tile: one persistent kernel runs every
   // iteration (cg_small.cu); otherwise graphs of K iterations.  Measured at
-  // p = 4: the persistent kernel is faster up to 32 x 32 (16^2: 1.80 against
+  // p = 4 with FP64 chains in both: the persistent kernel is faster up to 32 x 32 (16^2: 1.80 against
   // 2.2 ms), slower at 64 x 64 (12.2 against 9.9 ms: hundreds of CTAs meet at
   // each grid barrier)
   const bool small = sizeof(T) == 8 && is_pernode(op->cfg64, op->p) && op->dim <= kSmallCgDim;

@@ -118,6 +118,9 @@ double kappa_estimate(int p, int dim, double pen) {
   return c[p < 1 ? 1 : (p > 8 ? 8 : p)] * (double)dim * dim * scale;
 }
 
+// (Pairs for an ill-conditioned reliable-update solve: chosen when the FP64 apply
+// ran FP64 chains.  With the fixed-point one FP64 is the faster kind: 512^2, p = 6
+// 0.22 s against 0.75.)
 int choose_inner(int requested, int p, int dim, double pen) {
   if (requested == SIPG_INNER_F32 || requested == SIPG_INNER_PAIRS || requested == SIPG_INNER_F64) return requested;
   return kappa_estimate(p, dim, pen) * std::ldexp(1.0, -24) < 0.01 ? SIPG_INNER_F32 : SIPG_INNER_PAIRS;

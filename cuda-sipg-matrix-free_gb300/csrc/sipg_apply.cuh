@@ -103,13 +103,13 @@ struct KwInSmem {
 
 // Where a thread keeps its element's nodal block: only the owning thread
 // reads it (halo elements come from global memory, neighbours exchange face
-// values only), so where the n^2 values fit in registers -- FP32 up to p = 6
+// values only), so where the n^2 values fit in registers -- FP32 up to p = 7
 // (the row form, fully unrolled; measured: p = 4 426 -> 492 GDoF/s, p = 6
-// 316 -> 366) -- they stay there, and the tile's shared memory holds the
+// 316 -> 366; p = 7, 391^2 53.9 -> 41.5 us) -- they stay there, and the tile's shared memory holds the
 // faces alone.
 template <typename T, int P>
 struct NodalInRegs {
-  static constexpr bool value = sizeof(T) == 4 && P <= 7;
+  static constexpr bool value = P <= 7;
 };
 
 template <typename T, int P, int TX, int TY>
@@ -122,8 +122,8 @@ struct ApplySmem {
   static constexpr size_t bytes = (size_t)(US + XF + YF + KW) * sizeof(T);
 };
 
-// Phase-2 form per degree: the all-register form up to p = 6, the column form
-// beyond (whose n^2 outputs would not fit in registers).
+// Phase-2 form per degree: the all-register form up to p = 7, the column form
+// at p = 8 (whose n^2 outputs would not fit in registers).
 template <typename T, int P>
 struct ApplyColumnForm {
   static constexpr bool value = P >= 8;
@@ -210,7 +210,6 @@ __device__ __forceinline__ void apply_tile(const ApplyArgs<T>& a, const Tab<T, P
   // a smooth vector the FP32 operator's relative error falls from
   // ~kappa eps_32 (~1 at 512 x 512, p = 6) to ~dim eps_32, which is what an
   // FP32 inner solve needs to see the smooth modes.
-  constexpr bool kPivot = sizeof(T) == 4 || MODE != BASE;
   using S = ApplySmem<T, P, TX, TY>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ T red_sh[32];
@@ -282,18 +281,18 @@ __device__ __forceinline__ void apply_tile(const ApplyArgs<T>& a, const Tab<T, P
 #pragma unroll
     for (int j = 0; j < N1; ++j) {  // LEFT face of this element (x face slot tx)
       T d = T(0);
-      const T pv = kPivot ? U(0, j) : T(0);
+      const T pv = U(0, j);
 #pragma unroll
-      for (int i = 0; i < N1; ++i) d = fma(tb.D0[i], kPivot ? U(i, j) - pv : U(i, j), d);
+      for (int i = 0; i < N1; ++i) d = fma(tb.D0[i], U(i, j) - pv, d);
       XFr(ty, 0, j, tx) = U(0, j);
       XFr(ty, 1, j, tx) = d;
     }
 #pragma unroll
     for (int j = 0; j < N1; ++j) {  // DOWN face (y face slot ty+1)
       T d = T(0);
-      const T pv = kPivot ? U(j, 0) : T(0);
+      const T pv = U(j, 0);
 #pragma unroll
-      for (int i = 0; i < N1; ++i) d = fma(tb.D0[i], kPivot ? U(j, i) - pv : U(j, i), d);
+      for (int i = 0; i < N1; ++i) d = fma(tb.D0[i], U(j, i) - pv, d);
       YFr(ty + 1, 0, j, tx) = U(j, 0);
       YFr(ty + 1, 1, j, tx) = d;
     }
@@ -309,7 +308,7 @@ __device__ __forceinline__ void apply_tile(const ApplyArgs<T>& a, const Tab<T, P
         for (int i = 0; i < N1; ++i) {
           const T v = ld(j * N1 + i, he);
           if (i == 0) u0 = v;
-          d = fma(tb.D0[i], kPivot ? v - u0 : v, d);
+          d = fma(tb.D0[i], v - u0, d);
         }
         YFr(0, 0, j, t) = u0;
         YFr(0, 1, j, t) = d;
@@ -326,7 +325,7 @@ __device__ __forceinline__ void apply_tile(const ApplyArgs<T>& a, const Tab<T, P
         for (int i = 0; i < N1; ++i) {
           const T v = ld(i * N1 + j, he);
           if (i == 0) u0 = v;
-          d = fma(tb.D0[i], kPivot ? v - u0 : v, d);
+          d = fma(tb.D0[i], v - u0, d);
         }
         XFr(r, 0, j, TX) = u0;
         XFr(r, 1, j, TX) = d;
@@ -341,9 +340,9 @@ __device__ __forceinline__ void apply_tile(const ApplyArgs<T>& a, const Tab<T, P
 #pragma unroll
     for (int j = 0; j < N1; ++j) {
       T dN = T(0);
-      const T pv = kPivot ? U(0, j) : T(0);
+      const T pv = U(0, j);
 #pragma unroll
-      for (int i = 0; i < N1; ++i) dN = fma(tb.DN[i], kPivot ? U(i, j) - pv : U(i, j), dN);
+      for (int i = 0; i < N1; ++i) dN = fma(tb.DN[i], U(i, j) - pv, dN);
       const T u0 = rint ? XFr(ty, 0, j, tx + 1) : T(0);
       const T d0 = rint ? XFr(ty, 1, j, tx + 1) : T(0);
       T J, Q;
@@ -355,9 +354,9 @@ __device__ __forceinline__ void apply_tile(const ApplyArgs<T>& a, const Tab<T, P
 #pragma unroll
     for (int j = 0; j < N1; ++j) {
       T dN = T(0);
-      const T pv = kPivot ? U(j, 0) : T(0);
+      const T pv = U(j, 0);
 #pragma unroll
-      for (int i = 0; i < N1; ++i) dN = fma(tb.DN[i], kPivot ? U(j, i) - pv : U(j, i), dN);
+      for (int i = 0; i < N1; ++i) dN = fma(tb.DN[i], U(j, i) - pv, dN);
       const T u0 = uint_ ? YFr(ty, 0, j, tx) : T(0);
       const T d0 = uint_ ? YFr(ty, 1, j, tx) : T(0);
       T J, Q;
@@ -396,7 +395,7 @@ __device__ __forceinline__ void apply_tile(const ApplyArgs<T>& a, const Tab<T, P
           const T v = ld(j * N1 + i, he);
           if (i == 0) v0 = v;
           if (i == N) uN = v;
-          dN = fma(tb.DN[i], kPivot ? v - v0 : v, dN);
+          dN = fma(tb.DN[i], v - v0, dN);
         }
         T J, Q;
         combine(j, true, YFr(TY, 0, j, t), YFr(TY, 1, j, t), uN, dN, J, Q);
@@ -416,7 +415,7 @@ __device__ __forceinline__ void apply_tile(const ApplyArgs<T>& a, const Tab<T, P
           const T v = ld(i * N1 + j, he);
           if (i == 0) v0 = v;
           if (i == N) uN = v;
-          dN = fma(tb.DN[i], kPivot ? v - v0 : v, dN);
+          dN = fma(tb.DN[i], v - v0, dN);
         }
         T J, Q;
         combine(j, true, XFr(r, 0, j, 0), XFr(r, 1, j, 0), uN, dN, J, Q);
@@ -460,18 +459,18 @@ __device__ __forceinline__ void apply_tile(const ApplyArgs<T>& a, const Tab<T, P
         }
         T p0[N1];  // the x-sums' pivots u(0, j) (FP32)
 #pragma unroll
-        for (int j = 0; j < N1; ++j) p0[j] = kPivot ? Uv(0, j) : T(0);
+        for (int j = 0; j < N1; ++j) p0[j] = Uv(0, j);
 #pragma unroll
         for (int i = 0; i < N1; ++i) {
 #pragma unroll
           for (int j = 0; j < N1; ++j)
-            o[j] = fma(KWv((i1 * N1 + i) * N1 + j), kPivot ? Uv(i, j) - p0[j] : Uv(i, j), o[j]);
+            o[j] = fma(KWv((i1 * N1 + i) * N1 + j), Uv(i, j) - p0[j], o[j]);
         }
         T cp[N1];  // the row (i1, .), less its first value (FP32)
 #pragma unroll
         for (int i = 0; i < N1; ++i) c[i] = U(i1, i);
 #pragma unroll
-        for (int i = 0; i < N1; ++i) cp[i] = kPivot ? c[i] - c[0] : c[i];
+        for (int i = 0; i < N1; ++i) cp[i] = c[i] - c[0];
         const T gj = YFr(ty + 1, 0, i1, tx), hj = YFr(ty, 0, i1, tx);
 #pragma unroll
         for (int j = 0; j < N1; ++j) {
@@ -504,11 +503,9 @@ __device__ __forceinline__ void apply_tile(const ApplyArgs<T>& a, const Tab<T, P
         T r[N1];
 #pragma unroll
         for (int i = 0; i < N1; ++i) r[i] = U(i, j);
-        if (kPivot) {
-          const T r0 = r[0];
+        const T r0 = r[0];
 #pragma unroll
-          for (int i = 0; i < N1; ++i) r[i] = r[i] - r0;
-        }
+        for (int i = 0; i < N1; ++i) r[i] = r[i] - r0;
 #pragma unroll
         for (int i1 = 0; i1 < N1; ++i1) {
           T s = T(0);
@@ -523,11 +520,9 @@ __device__ __forceinline__ void apply_tile(const ApplyArgs<T>& a, const Tab<T, P
         T c[N1];
 #pragma unroll
         for (int i = 0; i < N1; ++i) c[i] = U(j, i);
-        if (kPivot) {
-          const T c0 = c[0];
+        const T c0 = c[0];
 #pragma unroll
-          for (int i = 0; i < N1; ++i) c[i] = c[i] - c0;
-        }
+        for (int i = 0; i < N1; ++i) c[i] = c[i] - c0;
 #pragma unroll
         for (int i2 = 0; i2 < N1; ++i2) {
           T s = T(0);

@@ -16,16 +16,16 @@
 // integers or through the chain of chain_node, so every tile shape gives the
 // same bits.
 //
-// Bound by integer issue and its latency: 183 instructions per DoF at p = 4 (29
+// Bound by integer issue and its latency: 180 instructions per DoF at p = 4 (29
 // of them the products; the rest conversions, parity form, limbs, 64-bit
-// additions and shared memory); ncu: multiply-add pipe 54 %, 46 % of the issue
+// additions and shared memory); ncu: multiply-add pipe 57 %, 46 % of the issue
 // slots with the 16 warps per SM that registers and shared memory allow, where FP64 chains are bound by an FP64
 // pipe of 2 operations per SM and cycle (21 per DoF).  Measured, FP64 chains
-// against this: 1024^2, p = 4 1080 -> 266 us (388 -> 1577 GB/s of the 16 bytes
-// per DoF); 443^2, p = 8 977 -> 288 us; ~16 M DoF, p = 1..8: 25, 26, 25, 24, 22,
-// 20, 18, 16 -> 81, 97, 94, 98, 79, 70, 67, 55 GDoF/s.  The error
-// against extended precision fell with it (p = 4, uniform values, relative
-// 2-norm: 2.8e-16 -> 1.1e-16).
+// against this: 1024^2, p = 4 1080 -> 262 us (388 -> 1604 GB/s of the 16 bytes
+// per DoF); 443^2, p = 8 977 -> 249 us; ~16 M DoF, p = 1..8: 25, 26, 25, 24, 22,
+// 20, 18, 16 -> 84, 104, 103, 95, 87, 77, 74, 64 GDoF/s.  The 2-norm error against
+// extended precision fell with it (p = 4, uniform values: 2.8e-16 -> 1.1e-16);
+// entry by entry see sipg_fx.cuh.
 #pragma once
 
 #include <type_traits>

@@ -9,8 +9,9 @@
 // coefficient is an integer held as two limbs,
 //     F = h 2^29 + l.
 // A product adds h h' to one 64-bit sum and h l' + l h' to another (three
-// IMAD.WIDE; l l' is left out, about 2^-57 of the largest product).  The sums
-// are exact, and a result is rounded once, on its way back to a double.
+// IMAD.WIDE; l l' is left out, up to half a unit of the total).  The kept products
+// are summed without rounding, so their order is free, and a result is rounded
+// once more on its way back to a double.
 //
 // The LGL nodes are symmetric, so every 1-D matrix here maps even functions
 // of the node index to even ones and odd to odd: values are kept as sums and
@@ -32,13 +33,15 @@
 // error on sin(2 pi x) sin(3 pi y), 12^2 elements, p = 4, penalty 100 p^2: 9.0e-14
 // with integer jumps, 1.4e-14 with FP64 ones, 1.8e-14 with FP64 chains.
 //
-// Accuracy.  A value's quantum is 2^-55 of the element's largest magnitude (a
-// value within 1/4 of it is exact), a coefficient's 2^-58 of the largest (the
-// tables are built in extended precision); a plain FP64 chain rounds each of
-// its 2n + 4 steps at 2^-53 of the partial sum.  Zero-sum rows (stiffness,
-// derivative) sum to zero exactly.  An element whose neighbour is more than
-// 2^kFxRoom times larger takes a coarser scale.
-//
+// Accuracy.  A value's quantum is 2^-55 of its element's scale (a value within 1/4
+// of the largest one is exact), a coefficient's 2^-58 of the largest (the tables
+// are built in extended precision), and a total's unit is 2^(3 - sk) of the scale
+// (sk: fx_scale; 2^-56, 2^-54, 2^-53, 2^-52, 2^-53, 2^-52, 2^-53, 2^-52 for p = 1..8), to which each
+// parity component is rounded and of which each dropped l l' is up to a half.  A
+// plain FP64 chain rounds each of its 2n + 4 steps at 2^-53 of the partial sum.  The
+// integer coefficients of a zero-sum row (stiffness, derivative) sum to zero; the
+// dropped products leave a constant's result within some units of zero.  An element
+// whose neighbour is more than 2^kFxRoom times larger takes a coarser scale.
 // That is accuracy relative to the element's (and its neighbours') largest
 // values.  An output sums its own row and column of the element, its face terms
 // and the traces across, and where those are all small, chains keep it accurate
@@ -49,8 +52,8 @@
 // beside non-zeros.  The others' entry-wise error is bounded by the scale;
 // against the sum of the entry's terms it reaches 900 2^-53 (a load vector,
 // whose corner nodes carry small weights, p = 8; chains: 4 2^-53), 15 2^-53 on
-// uniform values (chains 13).  CG directions, p = 1..8: 0.1 to 1.2 in 1000
-// elements lie beyond 2^-4, 3 to 30 beyond 2^-2.
+// uniform values (chains 13).  Of the elements of CG directions (means over a solve,
+// p = 2..8) 0.1 to 1.2 in 1000 lie beyond 2^-4, 9 to 29 beyond 2^-2.
 //
 // Range.  The scale is the element's own, so vectors of any magnitude keep
 // this accuracy.  An element with an infinity, a NaN, or a magnitude near the
@@ -340,7 +343,8 @@ __device__ __forceinline__ void fx_derivatives(const FxTab<P>& fx, int wb, Get g
 // Whether the penalty's coefficients nu HB(b) w_b, scaled as the tables, pass
 // 2^60: the integer terms of the largest jumps (components below 2^(kFxBits + 2),
 // times 2^kFxRoom from a larger neighbour, from two faces at a corner node) could
-// then pass 2^63 units.  (At a penalty of p^2 none does; from about 3 p^2 on.)
+// then pass 2^63 units: from penalties of 4.0, 1.5, 4.3, 2.8, 2.3, 1.8, 1.6 and 1.4
+// p^2 on for p = 1..8.
 __device__ __forceinline__ bool fx_large_nu(double nu_wmax, int sk) { return fx_biased(nu_wmax) - 1022 + sk > 60; }
 __device__ __forceinline__ int2 fx_nu(double wnu, int sk) {
   return fx_limbs_of(__double2ll_rn(wnu * __hiloint2double((1023 + sk) << 20, 0)));

@@ -113,9 +113,11 @@ enum ApplyMode : int {
   // differences from its element's first value (the FP32 apply always takes
   // them, from one value of the element line): the residual checks and outer steps of the mixed solvers,
   // where a smooth iterate's rounding in the plain sums would put a floor
-  // near 1e-10 under the true relative residual at 1024^2, p = 4.  The FP64
-  // sums themselves are exact (sipg_fx.cuh); what a difference saves is the
-  // value's rounding to 55 bits below the element's largest one.  The FP64
+  // near 1e-10 under the true relative residual at 1024^2, p = 4 (solved to 9.6e-11
+  // over differences, the plain sums say 1.6e-10).  The FP64 sums are integers
+  // (sipg_fx.cuh); a difference saves the value's rounding to 55 bits below the
+  // element's largest one.  Elements that take FP64 chains difference along the
+  // line, as FP32 does.  The FP64
   // CG and the plain apply keep the plain sums.  (The per-node FP64 tile of
   // small meshes runs the plain modes for these.)
   APPLY_RESID_PIVOT = 4,
@@ -165,8 +167,11 @@ struct TileCfg {
 __host__ __device__ constexpr int pernode_ey(int p) { return p == 1 ? 4 : 2; }
 __host__ __device__ constexpr int pernode_ex(int p, int shape) { return (p <= 2 ? 4 : 2) * (shape ? 2 : 1); }
 // FP64 operators up to kPernodeDefaultDim elements per edge start with the
-// per-node tile (measured faster than 32-element rows up to there), shape 1
-// above kPernodeWideDim
+// per-node tile, shape 1 above kPernodeWideDim.  The lines were drawn with FP64
+// chains in every tile.  With the fixed-point tiles, us of the per-node tile and
+// of 32 x 4 elements: p = 2, 64^2 6.4 and 8.3, 96^2 10.4 and 8.3; p = 4, 48^2 8.3
+// and 12.6, 64^2 10.5 and 12.5, 96^2 16.6 and 12.5, 128^2 26.8 and 12.6; p = 8, 48^2
+// 14.6 and 26.8, 64^2 24.4 and 25.0, 128^2 72 and 27
 constexpr int kPernodeDefaultDim = 128;
 constexpr int kPernodeWideDim = 32;
 inline bool is_pernode(const TileCfg& c, int p) { return c.tpe == (p + 1) * (p + 1); }
